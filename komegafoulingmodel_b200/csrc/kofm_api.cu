@@ -187,10 +187,16 @@ namespace {
         }                                                                         \
     } while (0)
 
+// Waits for the legacy default stream, on which the zero fills and the blocking
+// uploads below run: a context's own stream does not order itself after it, and
+// what the caller has queued there (another library's kernels) can hold those
+// fills back past the context's first kernels.
+int legacy_sync(int code) { return cudaStreamSynchronize(cudaStreamLegacy) == cudaSuccess ? KOFM_OK : code; }
+
 int dalloc(void** p, size_t bytes) {
     if (cudaMalloc(p, bytes) != cudaSuccess) return KOFM_ERR_BUFFER_ALLOCATION;
     if (cudaMemset(*p, 0, bytes) != cudaSuccess) return KOFM_ERR_BUFFER_ALLOCATION;
-    return KOFM_OK;
+    return legacy_sync(KOFM_ERR_BUFFER_ALLOCATION);
 }
 
 template <typename T>
@@ -828,6 +834,10 @@ int kofm_create(const kofm_desc* d, kofm_ctx** out) {
     // rec / dxrec_idx default to -1 (no record)
     cudaMemset(c->rec, 0xff, D * sizeof(int32_t));
     cudaMemset(c->dxrec_idx, 0xff, D * sizeof(int32_t));
+    if (int _s = legacy_sync(KOFM_ERR_BUFFER_ALLOCATION)) {
+        kofm_destroy(c);
+        return _s;
+    }
     c->stats.steps_per_lb = c->steps_per_lb;
     c->stats.dt = c->dt;
     *out = c;
@@ -942,6 +952,7 @@ int kofm_set_geometry(kofm_ctx* c, const int16_t* ntype, const double* wallD,
         }
         if (e != cudaSuccess) return fail(KOFM_ERR_MEMORY_COPY);
     }
+    if (legacy_sync(KOFM_ERR_MEMORY_COPY)) return fail(KOFM_ERR_MEMORY_COPY);
     c->have_geometry = true;
     return KOFM_OK;
 }
@@ -1128,6 +1139,7 @@ int kofm_set_shear(kofm_ctx* c, const int32_t* nodes, int32_t n_nodes, const dou
         KOFM_CUDA_TRY(cudaMemcpy(c->shear_idx, idx.data(), idx.size() * sizeof(int32_t), cudaMemcpyHostToDevice),
                       KOFM_ERR_MEMORY_COPY);
     }
+    if ((st = legacy_sync(KOFM_ERR_MEMORY_COPY))) return st;
     c->shear_n = n_nodes;
     c->shear_nbl = n_bl;
     return KOFM_OK;
