@@ -27,10 +27,8 @@ struct kofm_ctx;
 namespace kofm {
 int th_solver_alloc(kofm_ctx* c);
 int ko_solver_alloc(KoSystem* sys, GmresControl** ctl, double** part, unsigned int** bar,
-                    int* nblocks, int P, int ny, int K, int dev, int max_blocks);
-int ss_solver_alloc(double** part, int** lhint, int* nblocks, int* pstrips, int* prows, int nx,
-                    int ny, int K, int dev, int max_blocks);
-int sp_solver_alloc(kofm_ctx* c);
+                    int* nblocks, int P, int ny, int K, int dev, int max_blocks, bool basis);
+int ss_solver_alloc(kofm_ctx* c);
 void ko_system_free(KoSystem* s);
 static int ug_pull(kofm_ctx* c);
 static void ug_reset(kofm_ctx* c);
@@ -112,12 +110,12 @@ struct kofm_ctx {
     double* gpart = nullptr;          // solver partial sums
     unsigned int* bar = nullptr;      // grid barrier words
     int solver_blocks = 0;
-    // one-sweep-per-cycle solver (kofm_sstep.cuh): partial sums, grid and
-    // the strips of its powers and update sweeps
+    // two-sweep solver (kofm_sstep.cuh): partial sums (room for ss_maxu units a
+    // system), grid, and the row ranges of its strips
     double* spart = nullptr;
-    int* ss_lhint = nullptr;          // powers of a cycle's first round, per system
-    int ss_blocks = 0, ss_pstrips = 0, ss_prows = 0;
-    SsLaunch sp{};                    // the same solver as separate phase launches
+    int* ss_lhint = nullptr;          // powers of a cycle's first sweep, per system
+    int ss_blocks = 0, ss_maxu = 0, sp_gram_blocks = 0, sp_upd_blocks = 0, sp_resid_blocks = 0;
+    short ss_gram_rows[SS_MAXL + 2][SS_MAXL + 2] = {}, ss_upd_rows[SS_MAXL + 2][SS_MAXL + 2] = {};
     int ss_hint[2] = {0, 0};          // host copy of ss_lhint (first-round powers)
     // the k-omega update as a device-driven CUDA graph (kofm_stepgraph.inc)
     KoStepState* kst = nullptr;       // sub-stepping state (device)
@@ -125,7 +123,6 @@ struct kofm_ctx {
     cudaGraph_t ug = nullptr;
     cudaGraphExec_t ugx = nullptr;
     bool ug_pending = false;          // updates launched since the state was last read back
-    bool ug_devupd = false;           // the graph's assembly node takes dt as a device-updated parameter
     long long launches_host = 0;      // k-omega kernel launches the host loop made since set_state
     int steps_per_lb = 1;
     int time_since_change = 0;
@@ -794,12 +791,11 @@ int kofm_create(const kofm_desc* d, kofm_ctx** out) {
         ALLOC_FIELD(c->O, D);
         ALLOC_FIELD(c->S, 3 * D);
         ALLOC_FIELD(c->nut, D);
+        // (the form the entry points take: solver_form)
+        const bool basis = d->komega_full_cycle || d->komega_classic == 1;
         int s2 = ko_solver_alloc(c->sys, &c->ctl, &c->gpart, &c->bar, &c->solver_blocks,
-                                 c->P, d->ny, d->krylov_dim, c->dev, d->solver_max_blocks);
-        if (s2) { kofm_destroy(c); return s2; }
-        s2 = ss_solver_alloc(&c->spart, &c->ss_lhint, &c->ss_blocks, &c->ss_pstrips, &c->ss_prows,
-                             d->nx, d->ny, d->krylov_dim, c->dev, d->solver_max_blocks);
-        if (!s2) s2 = sp_solver_alloc(c);
+                                 c->P, d->ny, d->krylov_dim, c->dev, d->solver_max_blocks, basis);
+        if (!s2) s2 = ss_solver_alloc(c);
         if (s2) { kofm_destroy(c); return s2; }
         if (cudaMallocHost(&c->h_ctl, sizeof(GmresControl)) != cudaSuccess ||
             cudaMallocHost(&c->h_kst, sizeof(KoStepState)) != cudaSuccess) {

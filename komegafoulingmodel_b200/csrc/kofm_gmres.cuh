@@ -58,17 +58,17 @@ struct GmresSys {
     int vec_index_sum;  // sum over built vectors of their index k in the cycle
     int update_terms;   // sum over cycles of the update's coefficient count kk
     int inject;         // test hook: report a NaN residual at the first check
-    int lev;            // one-sweep cycle: powers computed so far in this cycle
-    int ext;            // one-sweep cycle: 1 = more powers needed before the cut
-    int powers;         // one-sweep cycle: powers computed (all rounds and cycles)
-    int lnext;          // one-sweep cycle: first-round powers chosen for the next cycle (0: none yet)
-    // one-sweep cycle run as separate phase launches: the restart whose
-    // vectors are in use (buffer parity), the levels of the pending powers
-    // round (lfrom + 1 .. lto), a finished cycle waiting for its update and
-    // residual sweeps, and the field write-back done
-    int rst, lfrom, lto, ready, written;
+    int lev;            // two-sweep cycle: levels of its last Gram sweep
+    int ext;            // two-sweep cycle: 1 = more powers needed before the cut
+    int powers;         // two-sweep cycle: powers computed (all rounds and cycles)
+    int lnext;          // two-sweep cycle: first-round powers chosen for the next cycle (0: none yet)
+    // two-sweep cycle: the restart whose residual is in use (0: b'), the levels
+    // of the pending Gram sweep (0: none), what the update sweep does
+    // (SsApply), a kept correction waiting for its residual sweep, and the
+    // field written
+    int rst, lto, bmode, ready, written;
     double rho0, norm_rhs, rinv, rho, prev_err;
-    double abytes;      // one-sweep cycle: algorithmic bytes per node of the sweeps so far
+    double abytes;      // two-sweep cycle: algorithmic bytes per node of the sweeps so far
     double s[KOFM_MAX_KRYLOV];   // 1 / ||u_j||
     double h[KOFM_MAX_KRYLOV];   // Gram-Schmidt coefficients for the next vector
     double xi[KOFM_MAX_KRYLOV];
@@ -83,7 +83,7 @@ struct GmresControl {
     int passes;       // grid sweeps performed
     int any_active;
     int ntrace;       // grid barriers recorded in trace
-    int any_ext;      // one-sweep cycle: a system asks for more powers
+    int any_ext;      // two-sweep cycle: a system asks for more powers
     int rounds;       // phase-launch solve: rounds run
     int launches;     // phase-launch solve: kernel launches of the solve
     int pad;

@@ -46,10 +46,8 @@ struct KoSystem {
     double* rhs = nullptr;    // [D] b' = b - A x0 (also the residual of restart 0)
     double* r = nullptr;      // [D] residual of restarts >= 1
     double* x = nullptr;     // [D] correction
-    double* V = nullptr;      // [K x D] Krylov basis (orthogonalised, unscaled; interleaved),
-                              // or the powers p_1 .. p_K of the one-sweep cycle
-    double* x2 = nullptr;     // [D] correction and residual of alternate restarts
-    double* r2 = nullptr;     //     (the one-sweep cycle's update reads one, writes the other)
+    double* V = nullptr;      // [K x D] Krylov basis (orthogonalised, unscaled; interleaved) of the
+                              // one-vector-per-sweep form; the other forms keep no basis
 };
 
 struct AsmParams {
@@ -72,7 +70,7 @@ struct AsmParams {
     int nx, ny, P;
     int rows;  // rows per warp strip chunk
     long long D;
-    double mu, dt;
+    double mu;
 };
 
 struct Fd3 {
@@ -349,9 +347,8 @@ __device__ __forceinline__ void km_wait() { asm volatile("cp.async.wait_group %0
 // a per-warp ring of KM_R slots in shared memory, copied with cp.async
 // KM_R - 1 steps ahead; each lane reads back only the elements it copied, so
 // the warp needs no barrier.
-template <typename FT = float, bool DEVDT = false>
-__global__ void __launch_bounds__(KM_WARPS * 32, KOFM_ASM_MINBLOCKS)
-komega_assemble_kernel(const AsmParams p, const double* dt_dev) {
+template <typename FT>
+__device__ __forceinline__ void km_assemble(const AsmParams& p, const double dt) {
     using CT = typename KoClosure<FT>::type;
     constexpr unsigned FULL = 0xffffffffu;
     extern __shared__ __align__(16) unsigned char km_smem[];
@@ -373,8 +370,6 @@ komega_assemble_kernel(const AsmParams p, const double* dt_dev) {
     const bool xl = lane == 0 || lane == 31;
     const bool icol = lane >= 1 && lane <= KM_W && gxu < nx;
     const int colb = ((cx >> 5) << 7) + (cx & 31);
-    double dt = p.dt;
-    if (DEVDT) dt = __ldg(dt_dev);
     const FT* pK = static_cast<const FT*>(p.K);
     const FT* pO = static_cast<const FT*>(p.O);
     const FT* pY = static_cast<const FT*>(p.wallD);
@@ -484,6 +479,12 @@ komega_assemble_kernel(const AsmParams p, const double* dt_dev) {
         t = tn;
     }
     km_wait<0>();
+}
+
+template <typename FT>
+__global__ void __launch_bounds__(KM_WARPS * 32, KOFM_ASM_MINBLOCKS)
+komega_assemble_kernel(const AsmParams p, const double dt) {
+    km_assemble<FT>(p, dt);
 }
 
 }  // namespace kofm

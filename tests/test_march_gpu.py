@@ -1,0 +1,69 @@
+"""The two-sweep solve at the edges of its strips, rings and level counts: the
+correction it leaves in the fields satisfies the assembled rows.
+
+The rows (kofm_debug_komega_rows) are FP64 and so are the fields of the FP64
+form, so the residual b' - A d of d = (field after) - (field before) can be
+formed on the host.  Bound: the solve stops at ||b' - A d|| <= relTol ||b'||
+(checked with b' - A d summed in another order: a factor 1.01), and d carries
+the rounding of the fields it was added to, at most eps ||(I + |N|) |field||| <=
+2.5 eps ||field|| with the off-diagonals' row sums below 1.5."""
+import numpy as np
+import pytest
+
+from komegafoulingmodel_b200 import Lattice, _abi, desc_default
+from komegafoulingmodel_b200 import geometry as G
+from tests.cases import komega_state, perturbed_state
+
+pytestmark = pytest.mark.gpu
+
+REL_TOL = 1.0e-11
+
+
+def _matvec(coef, x, ny, nx):
+    """A x with unit diagonal; coef [4, ny, nx] E, W, N, S; periodic in x."""
+    n = np.vstack([x[1:], np.zeros((1, nx))])
+    s = np.vstack([np.zeros((1, nx)), x[:-1]])
+    return x + coef[0] * np.roll(x, -1, 1) + coef[1] * np.roll(x, 1, 1) + coef[2] * n + coef[3] * s
+
+
+@pytest.mark.parametrize("form", [0, 2])
+@pytest.mark.parametrize("nx,ny,krylov", [
+    (4, 5, 10),      # a strip wraps around the channel many times
+    (31, 18, 10), (200, 9, 10),           # narrower than a strip: wraps on both sides
+    (236, 12, 10), (237, 12, 10),         # one strip of 10 levels exactly, and one column more
+    (256, 34, 10), (257, 34, 10),         # one block's columns, and one more
+    (480, 21, 8), (481, 21, 8),           # two strips of 8 levels
+    (610, 66, 9), (1001, 130, 7),         # not multiples of anything
+    (300, 40, 1), (300, 40, 2), (300, 40, 3), (300, 40, 4), (300, 40, 5), (300, 40, 6),
+    (2100, 300, 10),                      # several units a block of the one-launch form
+])
+def test_solved_fields_satisfy_the_rows(kofm_lib, form, nx, ny, krylov):
+    ch = G.straight_channel(nx, ny)
+    f = perturbed_state(ch, seed=3, u_mean=0.05, rho_amp=1e-4, u_amp=5e-3, neq_amp=1e-5)
+    k, o, nut, s = komega_state(ch, seed=4)
+    d = desc_default()
+    d.nx, d.nx_full, d.ny = nx, nx, ny
+    d.tau, d.fterm, d.mu = 1.0 / (3 * 1e-3 + 0.5), 1e-7, 1e-3
+    d.use_komega, d.storage = 1, _abi.STORE_FP64
+    d.komega_rel_tol, d.komega_abs_tol = REL_TOL, 0.0
+    d.krylov_dim, d.komega_classic = krylov, form
+    d.komega_max_iters = 10000
+    with Lattice(d) as L:
+        L.set_geometry(ch.ntype, ch.wallD, ch.dX)
+        L.set_state(f, k, o, nut, s)
+        L.lb_step()
+        for _ in range(2):  # the second solve starts from the first one's cycle lengths
+            L.komega_assemble(1.0)
+            before = L.get_state()
+            rows = [L.komega_rows(i) for i in range(2)]
+            status, _, _ = L.komega_solve(raise_on_error=False)
+            after = L.get_state()
+            assert status == 0
+            for (coef, rhs), x0, x1 in zip(rows, (before[2], before[1]), (after[2], after[1])):
+                coef, rhs = coef.reshape(4, ny, nx), rhs.reshape(ny, nx)
+                x0, x1 = x0.reshape(ny, nx), x1.reshape(ny, nx)
+                fl = ch.fluid_mask()
+                r = (rhs - _matvec(coef, (x1 - x0) * fl, ny, nx)) * fl
+                bound = 1.01 * REL_TOL * np.linalg.norm(rhs) + 2.5 * np.finfo(float).eps * np.linalg.norm(x1)
+                assert np.abs(coef).sum(0).max() < 1.5
+                assert np.linalg.norm(r) <= bound, (np.linalg.norm(r), bound)
