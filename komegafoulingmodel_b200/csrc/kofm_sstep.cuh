@@ -62,7 +62,7 @@ struct SsArgs {
     int f64;
     const int16_t* ntype;
     GmresControl* ctl;
-    double* part;             // partial sums [2 SS_NG][maxu] (slot-major, one per unit)
+    double* part;             // partial sums [2][maxu][SS_NG] (a unit's sums side by side)
     int maxu;
     GridBarrier* bar;
     SsQueue* queue;
@@ -102,7 +102,7 @@ constexpr double SS_PIVOT_MIN = 1.0e-9;
 // magnitudes of its terms (the Gram entries' own sums over the nodes).
 constexpr double SS_PRED_EPS = 1.0e-13;
 
-// Sum over the first 16 lanes (every one of them gets it).
+// Sum over each half of a warp (every lane of the half gets it).
 __device__ __forceinline__ double ss_sum16(double x) {
 #pragma unroll
     for (int off = 8; off > 0; off >>= 1) x += __shfl_xor_sync(0xffffffffu, x, off);
@@ -150,7 +150,8 @@ __device__ __forceinline__ void ss_rank(SsCycleSmem& cs, int n) {
 // first vector that the reference's tests refuse (GMRESSolver.cpp:300-330):
 // diag(R) below rel_tol R(0, 0), or |xi_k| >= rho.  Latency-bound: a chain of a
 // shift, one product with G, two sums over the lanes and a square root per
-// vector.
+// vector.  The warp's halves do the same work, so that every lane holds what
+// the tests read.
 struct SsCycle {
     double V[SS_MAXL];  // this lane's coefficient of v_0 .. v_{built-1}
     int built;          // vectors built
@@ -158,7 +159,7 @@ struct SsCycle {
 };
 __device__ __forceinline__ void ss_cycle(SsCycle& c, SsCycleSmem& cs, int L, int K, double rel_tol, double rinv) {
     const unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 15;
     const int n = L + 1;
     double g[SS_MAXL + 1], GV[SS_MAXL];
 #pragma unroll
@@ -171,7 +172,7 @@ __device__ __forceinline__ void ss_cycle(SsCycle& c, SsCycleSmem& cs, int L, int
         if (k >= L || k >= K || c.cut) break;
         // w = A z, z = r / rho0 = rinv p_0 (k = 0) or v_{k-1}
         const double z = k == 0 ? (lane == 0 ? rinv : 0.0) : c.V[k > 0 ? k - 1 : 0];
-        const double zm = __shfl_up_sync(FULL, z, 1);
+        const double zm = __shfl_up_sync(FULL, z, 1, 16);
         double w = lane < n ? (lane == 0 ? z : z + zm) : 0.0;
         double a0 = 0.0, a1 = 0.0;
 #pragma unroll
@@ -194,7 +195,7 @@ __device__ __forceinline__ void ss_cycle(SsCycle& c, SsCycleSmem& cs, int L, int
         const double nk = nk2 > 0.0 ? nk2 * inv : 0.0;
         c.V[k] = w * inv;
         GV[k] = Gw * inv;
-        const double xi = rinv * __shfl_sync(FULL, GV[k], 0);  // <r / rho0, v_k>
+        const double xi = rinv * __shfl_sync(FULL, GV[k], 0, 16);  // <r / rho0, v_k>
         if (k == 0) r00 = nk;
         if (lane == 0) {
 #pragma unroll
@@ -205,8 +206,8 @@ __device__ __forceinline__ void ss_cycle(SsCycle& c, SsCycleSmem& cs, int L, int
         }
         c.built = k + 1;
         const double x = fabs(xi);
-        if (__shfl_sync(FULL, nk < rel_tol * r00 ? 1 : 0, 0)) c.cut = 1;
-        else if (__shfl_sync(FULL, x >= rho ? 1 : 0, 0)) c.cut = 2;
+        if (nk < rel_tol * r00) c.cut = 1;
+        else if (x >= rho) c.cut = 2;
         else {
             rho = sqrt((rho - x) * (rho + x));  // rho sin(acos(xi / rho))
             if (k == K - 1) c.cut = 3;
@@ -216,18 +217,18 @@ __device__ __forceinline__ void ss_cycle(SsCycle& c, SsCycleSmem& cs, int L, int
     __syncwarp();
 }
 
-// Start of a system's serial step after a Gram sweep of L levels, one warp: t
-// holds G(i, j) of p_0 .. p_L (slots ss_gslot).  Restart 0's first sweep also
-// takes the restart-0 convergence test from G(0, 0) = ||b'||^2
+// Start of a system's serial step after a Gram sweep of L levels, every second
+// warp: t holds G(i, j) of p_0 .. p_L (slots ss_gslot).  Restart 0's first
+// sweep also takes the restart-0 convergence test from G(0, 0) = ||b'||^2
 // (GMRESSolver::solve's checkConvergence).
 __device__ __forceinline__ void ss_gram_begin(const SsArgs& a, GmresSys& S, const double* t, int L, SsCycleSmem& cs) {
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, part = threadIdx.x >> 6;
     const int n = L + 1;
-    for (int e = lane; e < n * n; e += 32) {
+    for (int e = lane + 32 * part; e < n * n; e += 16 * SS_WARPS) {
         const int i = e / n, j = e - i * n;
         cs.G[e] = t[i <= j ? ss_gslot(i, j) : ss_gslot(j, i)];
     }
-    if (lane == 0) {
+    if (part == 0 && lane == 0) {
         const double rho0 = sqrt(t[0]);
         S.powers += L;
         if (S.restarts == 0) {
@@ -247,7 +248,6 @@ __device__ __forceinline__ void ss_gram_begin(const SsArgs& a, GmresSys& S, cons
             S.rinv = 1.0 / rho0;
         }
     }
-    __syncwarp();
 }
 
 // End of the serial step: the cut, the update coefficients on p_0 .. p_L into
@@ -365,6 +365,19 @@ __device__ __forceinline__ void ss_resid_step(const SsArgs& a, GmresSys& S, int 
     if (!S.active) S.bmode = SS_B_WRITE;
 }
 
+// (the words in flight and their arrival are separate, so that other loads can
+// be issued between)
+struct SsSysWord {
+    static constexpr int NW = (int)(sizeof(GmresSys) / 8);
+    unsigned long long w;
+    __device__ __forceinline__ void load(const GmresControl* ctl, int s) {
+        static_assert(NW <= SS_THREADS && sizeof(GmresSys) % 8 == 0, "one word a thread");
+        if ((int)threadIdx.x < NW) w = __ldcg(reinterpret_cast<const unsigned long long*>(&ctl->sys[s]) + threadIdx.x);
+    }
+    __device__ __forceinline__ void put(GmresSys& dst) const {
+        if ((int)threadIdx.x < NW) reinterpret_cast<unsigned long long*>(&dst)[threadIdx.x] = w;
+    }
+};
 __device__ __forceinline__ void sp_sys_load(const GmresControl* ctl, int s, GmresSys& dst) {
     constexpr int NW = (int)(sizeof(GmresSys) / 8);
     const unsigned long long* src = reinterpret_cast<const unsigned long long*>(&ctl->sys[s]);
@@ -939,9 +952,14 @@ __device__ __forceinline__ void ss_warp_sums(const double (&v)[N], int lane, F p
     }
 }
 
-// Sums of N per-thread values over the block into part[(base + k) * stride + at].
+// A unit's sums of system s.
+__device__ __forceinline__ double* ss_part(const SsArgs& a, int s, int unit) {
+    return a.part + ((long long)s * a.maxu + unit) * SS_NG;
+}
+
+// Sums of N per-thread values over the block into part[0 .. N).
 template <int N>
-__device__ __forceinline__ void ss_block_sums(const double (&v)[N], double* part, long long stride, int base, int at) {
+__device__ __forceinline__ void ss_block_sums(const double (&v)[N], double* part) {
     SsSmem& sm = ss_sm();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     ss_warp_sums<N, 16>(v, lane, [&](int k, double x) { sm.red[warp][k] = x; });
@@ -950,26 +968,65 @@ __device__ __forceinline__ void ss_block_sums(const double (&v)[N], double* part
         double x = 0.0;
 #pragma unroll
         for (int w = 0; w < SS_WARPS; ++w) x += sm.red[w][k];
-        part[(long long)(base + k) * stride + at] = x;
+        part[k] = x;
     }
     ss_sync_march();
 }
 
-// Sum of n values in a fixed order, one warp, every lane the result.
+// Sum of n units' first value in a fixed order, one warp, every lane the result.
 __device__ __forceinline__ double ss_sum_warp(const double* p, int n) {
-    const int lane = threadIdx.x & 31;
-    double v[4] = {0.0, 0.0, 0.0, 0.0};
-    int b = lane;
-    for (; b + 96 < n; b += 128)
-#pragma unroll
-        for (int k = 0; k < 4; ++k) v[k] += __ldcg(p + b + 32 * k);
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-        if (b + 32 * k < n) v[k] += __ldcg(p + b + 32 * k);
-    double x = (v[0] + v[1]) + (v[2] + v[3]);
+    double x = 0.0;
+    for (int b = threadIdx.x & 31; b < n; b += 32) x += __ldcg(p + (long long)b * SS_NG);
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) x += __shfl_xor_sync(0xffffffffu, x, off);
     return x;
+}
+
+// tot[s][k]: sums over the units, in a fixed order, of both systems' Gram
+// entries.  Warp w takes the units w, w + 8, ..; lane l of it the entries
+// l, l + 32, l + 64; then the warps' sums are added up.  A chain of waits for
+// L2: SS_SUM_U units of both systems are in flight at a time (one warp per
+// entry, its lanes across the units, waited for L2 and for a sum over the lanes
+// once per entry: 9 to 13 thousand cycles at 45 entries of 70 to 140 units,
+// where this takes 2 to 3).
+constexpr int SS_SUM_U = 5;
+__device__ __forceinline__ void ss_unit_sums(const SsArgs& a, const int (&ng)[2], const int (&n)[2], double (*tot)[SS_NG]) {
+    constexpr int C = (SS_NG + 31) / 32;
+    double(*red)[2 * SS_NG] = reinterpret_cast<double(*)[2 * SS_NG]>(ss_dyn);  // the march has ended
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double v[2][C] = {};
+    for (int b = warp; b < n[0] || b < n[1]; b += SS_WARPS * SS_SUM_U) {
+        double x[SS_SUM_U][2][C];
+#pragma unroll
+        for (int i = 0; i < SS_SUM_U; ++i)
+#pragma unroll
+            for (int s = 0; s < 2; ++s)
+#pragma unroll
+                for (int c = 0; c < C; ++c) {
+                    const int u = b + i * SS_WARPS, k = lane + 32 * c;
+                    x[i][s][c] = u < n[s] && k < ng[s] ? __ldcg(ss_part(a, s, u) + k) : 0.0;
+                }
+#pragma unroll
+        for (int i = 0; i < SS_SUM_U; ++i)
+#pragma unroll
+            for (int s = 0; s < 2; ++s)
+#pragma unroll
+                for (int c = 0; c < C; ++c) v[s][c] += x[i][s][c];
+    }
+#pragma unroll
+    for (int s = 0; s < 2; ++s)
+#pragma unroll
+        for (int c = 0; c < C; ++c)
+            if (lane + 32 * c < ng[s]) red[warp][SS_NG * s + lane + 32 * c] = v[s][c];
+    ss_sync_march();
+    for (int k = threadIdx.x; k < 2 * SS_NG; k += SS_THREADS) {
+        const int s = k / SS_NG, e = k - s * SS_NG;
+        if (e >= ng[s]) continue;
+        double x = 0.0;
+#pragma unroll
+        for (int w = 0; w < SS_WARPS; ++w) x += red[w][k];
+        tot[s][e] = x;
+    }
 }
 
 // Levels of the Gram sweep of system s (-1: none pending).
@@ -987,7 +1044,7 @@ __device__ __forceinline__ void ss_gram_march(const SsArgs& a) {
     double acc[NG];
     ss_march<L, true, J, float>(a, acc);
     const SsUnit& u = ss_sm().u;
-    ss_block_sums<NG>(acc, a.part, a.maxu, SS_NG * u.s + J * (J + 1) / 2, u.n);
+    ss_block_sums<NG>(acc, ss_part(a, u.s, u.n) + J * (J + 1) / 2);
 }
 // Unit n of the Gram sweep, and of the update sweep.  One unit per block: a
 // loop over units around this switch made the compiler keep (and spill)
@@ -1012,20 +1069,21 @@ __device__ __forceinline__ void ss_gram_serial(const SsArgs& a) {
     __shared__ double tot[2][SS_NG];
     __shared__ GmresSys sS[2];
     __shared__ SsCycleSmem cs[2];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    sp_sys_load(a.ctl, 0, sS[0]);
-    sp_sys_load(a.ctl, 1, sS[1]);
-    int ng[2];
-    for (int s = 0; s < 2; ++s) ng[s] = pl.lev[s] > 0 ? (pl.lev[s] + 1) * (pl.lev[s] + 2) / 2 : 0;
-    for (int i = warp; i < ng[0] + ng[1]; i += SS_WARPS) {
-        const int s = i < ng[0] ? 0 : 1, k = i - s * ng[0];
-        const double v = ss_sum_warp(a.part + (long long)(SS_NG * s + k) * a.maxu, pl.strips[s] * pl.rows);
-        if (lane == 0) tot[s][k] = v;
+    const int warp = threadIdx.x >> 5;
+    SsSysWord w[2];
+    int ng[2], n[2];
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+        w[s].load(a.ctl, s);
+        ng[s] = pl.lev[s] > 0 ? (pl.lev[s] + 1) * (pl.lev[s] + 2) / 2 : 0;
+        n[s] = ng[s] ? pl.strips[s] * pl.rows : 0;
     }
+    ss_unit_sums(a, ng, n, tot);
+    for (int s = 0; s < 2; ++s) w[s].put(sS[s]);
     ss_sync_march();
     const int s = warp & 1, L = pl.lev[s];
-    if (warp < 2 && L > 0) {
-        if (lane == 0)  // p_0 and the coefficients of the sweep, per node
+    if (L > 0) {
+        if (threadIdx.x == 32 * s)  // p_0 and the coefficients of the sweep, per node
             sS[s].abytes += 40.0 * pl.parts[s];
         ss_gram_begin(a, sS[s], tot[s], L, cs[s]);
     }
@@ -1152,7 +1210,7 @@ __device__ __forceinline__ bool ss_resid_units(const SsArgs& a, const bool act[2
             __stcg(reinterpret_cast<double2*>(S.r + g), make_double2(rr[0], rr[1]));
             acc[0] += rr[0] * rr[0] + rr[1] * rr[1];
         }
-        ss_block_sums<1>(acc, a.part, a.maxu, SS_NG * s, blockIdx.x);
+        ss_block_sums<1>(acc, ss_part(a, s, blockIdx.x));
     }
     return act[0] || act[1];
 }
@@ -1164,7 +1222,7 @@ __device__ __forceinline__ void ss_resid_serial(const SsArgs& a, const bool act[
     sp_sys_load(a.ctl, 1, sS[1]);
     const int warp = threadIdx.x >> 5;
     if (warp < 2 && act[warp]) {
-        const double v = ss_sum_warp(a.part + (long long)SS_NG * warp * a.maxu, gridDim.x);
+        const double v = ss_sum_warp(ss_part(a, warp, 0), gridDim.x);
         if ((threadIdx.x & 31) == 0) tot[warp] = v;
     }
     ss_sync_march();
