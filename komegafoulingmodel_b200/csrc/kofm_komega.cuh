@@ -98,17 +98,22 @@ __device__ __forceinline__ double dmaxr(double a, double b) { return a < b ? b :
 __device__ __forceinline__ double dminr(double a, double b) { return b < a ? b : a; }
 
 // Warp strips: KM_W interior columns per warp (lanes 1..30; lanes 0 and 31
-// are the ring), KM_WARPS independent warps per block, KOFM_ASM_ROWS rows per
-// warp (each chunk re-evaluates the closure of the ring rows above and below
-// it: 2 of KOFM_ASM_ROWS + 2 rows).
+// are the ring), KM_WARPS independent warps per block, a chunk of rows per
+// warp (which re-evaluates the closure of the ring rows above and below it).
+//
+// Rows of a chunk: as many as make one wave of resident warps, KM_ROWS_MIN to
+// KM_ROWS_MAX.  A warp goes through its rows one after the other, so on a small
+// lattice the chunk's length is the kernel's time; on a large one short chunks
+// evaluate more ring rows.  Whole steps, us, with chunks of 2 / 4 / 8 / 16 / 32
+// rows: 256x64 69.5 / 71.6 / 76.0 / 83.9 / 100.5, 1001x253 106 / 101 / 103 /
+// 109 / 127, 2048x256 181 / 180 / 181 / 187 / 201, 4096x512 459 / 443 / 436 /
+// 433 / 427, 16384x1024 2995 / 2853 / 2793 / 2773 / 2770.
 constexpr int KM_W = 30;
 #ifndef KOFM_ASM_WARPS
 #define KOFM_ASM_WARPS 4
 #endif
 constexpr int KM_WARPS = KOFM_ASM_WARPS;
-#ifndef KOFM_ASM_ROWS
-#define KOFM_ASM_ROWS 16
-#endif
+constexpr int KM_ROWS_MIN = 2, KM_ROWS_MAX = 32;
 #ifndef KOFM_ASM_MINBLOCKS
 #define KOFM_ASM_MINBLOCKS 4  // resident blocks per SM the register budget is set for
 #endif
@@ -328,6 +333,17 @@ enum { KF_K, KF_O, KF_KX, KF_OX, KF_Y, KF_R, KF_N, KF_U, KF_V, KF_SA, KF_SB, KF_
 template <typename FT>
 constexpr size_t km_smem_bytes() { return sizeof(FT) * KM_WARPS * KM_R * KM_NF * 32; }
 
+// Warps of an assembly: one per strip and chunk of rows.
+__host__ __device__ __forceinline__ int km_warps(const AsmParams& p) {
+    return ((p.nx + KM_W - 1) / KM_W) * ((p.ny + p.rows - 1) / p.rows);
+}
+inline int km_rows(int nx, int ny, int sms) {
+    const int strips = (nx + KM_W - 1) / KM_W, wave = sms * KOFM_ASM_MINBLOCKS * KM_WARPS;
+    const int chunks = wave / strips < 1 ? 1 : wave / strips;
+    const int rows = (ny + chunks - 1) / chunks;
+    return rows < KM_ROWS_MIN ? KM_ROWS_MIN : rows > KM_ROWS_MAX ? KM_ROWS_MAX : rows;
+}
+
 template <typename FT>
 __device__ __forceinline__ void km_cp(FT* dst, const FT* src) {
     const unsigned sa = (unsigned)__cvta_generic_to_shared(dst);
@@ -355,9 +371,8 @@ __device__ __forceinline__ void km_assemble(const AsmParams& p, const double dt)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int nx = p.nx, ny = p.ny;
     const int nstrips = (nx + KM_W - 1) / KM_W;
-    const int nchunks = (ny + p.rows - 1) / p.rows;
     const int wid = blockIdx.x * KM_WARPS + warp;
-    if (wid >= nstrips * nchunks) return;  // whole warps
+    if (wid >= km_warps(p)) return;  // whole warps
     const int x0 = (wid % nstrips) * KM_W;
     const int y0 = (wid / nstrips) * p.rows;
     const int y1 = min(ny, y0 + p.rows);

@@ -86,3 +86,32 @@ def test_assembly_rows_match_oracle(kofm_lib, oracle, storage, tol, dt):
         print(name, storage, dt, e_coef, e_rhs)
         assert e_coef < tol and e_rhs < tol, (name, e_coef, e_rhs)
         assert np.all(coef[:, ~fl] == 0.0) and np.all(rhs[~fl] == 0.0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("ny,repeat", [(253, 17), (253, 30), (260, 137), (3, 40)])
+def test_chunk_length_does_not_change_the_rows(kofm_lib, ny, repeat):
+    """A warp's chunk of rows grows with the lattice (2 to 32 rows; on 148 SMs
+    here 4, 7, 32 and 2, each but the last with a shorter chunk at the end).  A
+    state of period 60 in x, assembled once on 60 columns (2 rows a chunk) and
+    once on `repeat` times as many: the same numbers at every node."""
+    nx, mu = 60, 5e-4
+    ch = G.straight_channel(nx, ny)
+    state = (perturbed_state(ch, seed=3, u_mean=0.03), *komega_state(ch, seed=4, k0=4e-5, o0=2e-3, s_amp=2e-4))
+    out = []
+    for m in (1, repeat):
+        wide = G.straight_channel(nx * m, ny)
+        d = desc_default()
+        d.nx, d.nx_full, d.ny = nx * m, nx * m, ny
+        d.tau, d.fterm, d.mu = 1.0 / (3 * mu + 0.5), 0.0, mu
+        d.use_komega = 1
+        with Lattice(d) as L:
+            L.set_geometry(wide.ntype, wide.wallD, wide.dX)
+            L.set_state(*[np.tile(np.reshape(a, (-1, ny, nx)), (1, 1, m)) for a in state])
+            L.lb_step()
+            L.komega_assemble(1.0)
+            out.append([np.concatenate([c.reshape(4, ny, nx * m), r.reshape(1, ny, nx * m)])
+                        for c, r in map(L.komega_rows, range(2))])
+    for one, many in zip(*out):
+        assert np.isfinite(one).all() and np.any(one)
+        assert np.array_equal(np.tile(one, (1, 1, repeat)), many)
