@@ -331,7 +331,9 @@ static_assert((KM_R & (KM_R - 1)) == 0 && KM_R >= 2, "ring depth: a power of two
 enum { KF_K, KF_O, KF_KX, KF_OX, KF_Y, KF_R, KF_N, KF_U, KF_V, KF_SA, KF_SB, KF_SC, KM_NF };
 
 template <typename FT>
-constexpr size_t km_smem_bytes() { return sizeof(FT) * KM_WARPS * KM_R * KM_NF * 32; }
+constexpr size_t km_ring_bytes() { return sizeof(FT) * KM_R * KM_NF * 32; }  // a warp's
+template <typename FT>
+constexpr size_t km_smem_bytes() { return KM_WARPS * km_ring_bytes<FT>(); }
 
 // Warps of an assembly: one per strip and chunk of rows.
 __host__ __device__ __forceinline__ int km_warps(const AsmParams& p) {
@@ -364,14 +366,13 @@ __device__ __forceinline__ void km_wait() { asm volatile("cp.async.wait_group %0
 // KM_R - 1 steps ahead; each lane reads back only the elements it copied, so
 // the warp needs no barrier.
 template <typename FT>
-__device__ __forceinline__ void km_assemble(const AsmParams& p, const double dt) {
+__device__ __forceinline__ void km_assemble(const AsmParams& p, const double dt, const int wid) {
     using CT = typename KoClosure<FT>::type;
     constexpr unsigned FULL = 0xffffffffu;
     extern __shared__ __align__(16) unsigned char km_smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int nx = p.nx, ny = p.ny;
     const int nstrips = (nx + KM_W - 1) / KM_W;
-    const int wid = blockIdx.x * KM_WARPS + warp;
     if (wid >= km_warps(p)) return;  // whole warps
     const int x0 = (wid % nstrips) * KM_W;
     const int y0 = (wid / nstrips) * p.rows;
@@ -499,7 +500,7 @@ __device__ __forceinline__ void km_assemble(const AsmParams& p, const double dt)
 template <typename FT>
 __global__ void __launch_bounds__(KM_WARPS * 32, KOFM_ASM_MINBLOCKS)
 komega_assemble_kernel(const AsmParams p, const double dt) {
-    km_assemble<FT>(p, dt);
+    km_assemble<FT>(p, dt, blockIdx.x * KM_WARPS + (threadIdx.x >> 5));
 }
 
 }  // namespace kofm

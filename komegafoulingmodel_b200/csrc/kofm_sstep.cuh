@@ -1027,6 +1027,8 @@ __device__ __forceinline__ void ss_unit_sums(const SsArgs& a, const int (&ng)[2]
         for (int w = 0; w < SS_WARPS; ++w) x += red[w][k];
         tot[s][e] = x;
     }
+    // (bulk copies of a later unit write here)
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
 // Levels of the Gram sweep of system s (-1: none pending).
@@ -1310,20 +1312,23 @@ __device__ __forceinline__ void ss_specialise(const SsArgs& a, F body) {
     ss_sync_block();
 }
 
+// (returns the rounds run)
 template <typename FT>
-__device__ __forceinline__ void ss_solve(const SsArgs& a) {
+__device__ __forceinline__ int ss_solve(const SsArgs& a) {
     if (blockIdx.x == 0 && threadIdx.x == 0) __stcg(&a.ctl->t_start, globaltimer_ns());
     // every restart takes at most two rounds (its first and one extension)
-    for (int round = 0; round < 2 * a.max_restarts + 2; ++round) {
+    int round = 0;
+    while (round < 2 * a.max_restarts + 2) {
+        ++round;
         {
             bool act[2];
             ss_resid_pending(a, act);
-            if (ss_resid_units(a, act) && !ss_sync(a, [&] { ss_resid_serial(a, act); })) return;
+            if (ss_resid_units(a, act) && !ss_sync(a, [&] { ss_resid_serial(a, act); })) return round;
         }
         {
             if (ss_begin(a, true, ss_gram_levels(a, 0), ss_gram_levels(a, 1))) {
                 for (int n = blockIdx.x; n < ss_sm().plan.total; n += gridDim.x) ss_gram_unit(a, n);
-                if (!ss_sync(a, [&] { ss_gram_serial(a); })) return;
+                if (!ss_sync(a, [&] { ss_gram_serial(a); })) return round;
             }
         }
         {
@@ -1331,9 +1336,10 @@ __device__ __forceinline__ void ss_solve(const SsArgs& a) {
                 for (int n = blockIdx.x; n < ss_sm().plan.total; n += gridDim.x) ss_upd_unit<FT>(a, n);
             ss_write_units<FT>(a);
         }
-        if (!ldc(&a.ctl->any_active)) return;
-        if (!ss_sync(a, [&] { if (threadIdx.x == 0) ss_upd_serial(a); })) return;
+        if (!ldc(&a.ctl->any_active)) return round;
+        if (!ss_sync(a, [&] { if (threadIdx.x == 0) ss_upd_serial(a); })) return round;
     }
+    return round;
 }
 
 template <typename FT>
@@ -1378,20 +1384,25 @@ struct KoStepState {
     int fail_mask;
     int substeps;          // solves of the last update
     int launches;          // kernel launches of the last update
-    int fresh;             // 1: the next body starts an update (doubling test not yet applied)
+    int fresh;             // 1: the next sub-step is an update's first (doubling test not yet applied)
     int again;             // 1: the running solve needs another round (no assembly)
+    int go;                // 1: the running update is not finished
     long long updates;     // updates run since the last reset
     long long launches_total;  // kernel launches of all updates since the last reset
 };
 
 // Control block of a solve: both systems iterating, restart 0, first sweep of
 // l0 / l1 levels, a pending failure injection (kofm_debug_fail_solves).
+// (MARCH: by the marching threads of a block whose grid is at its barriers)
+template <bool MARCH>
 __device__ __forceinline__ void ss_ctl_init(GmresControl* ctl, GridBarrier* bar, SsQueue* queue, KoStepState* st,
                                             int l0, int l1) {
     constexpr int NW = (int)(sizeof(GmresControl) / sizeof(unsigned int));
     unsigned int* w = reinterpret_cast<unsigned int*>(ctl);
-    for (int i = threadIdx.x; i < NW; i += blockDim.x) w[i] = 0u;
-    __syncthreads();
+    const int threads = MARCH ? SS_THREADS : (int)blockDim.x;
+    for (int i = threadIdx.x; i < NW; i += threads) w[i] = 0u;
+    if (MARCH) ss_sync_march();
+    else __syncthreads();
     if (threadIdx.x == 0) {
         int inject = 0;
         if (st->fail_solves > 0) {
@@ -1405,14 +1416,16 @@ __device__ __forceinline__ void ss_ctl_init(GmresControl* ctl, GridBarrier* bar,
         }
         ctl->any_active = 1;
         ctl->t_start = globaltimer_ns();
-        bar->count = 0u;
-        bar->gen = 0u;
-        queue->count = 0u;
+        if (!MARCH) {
+            bar->count = 0u;
+            bar->gen = 0u;
+            queue->count = 0u;
+        }
     }
 }
 
 __global__ void sp_init_kernel(GmresControl* ctl, GridBarrier* bar, SsQueue* queue, KoStepState* st, int l0, int l1) {
-    ss_ctl_init(ctl, bar, queue, st, l0, l1);
+    ss_ctl_init<false>(ctl, bar, queue, st, l0, l1);
 }
 
 // (st: the sub-stepping state of the update graph, whose sweeps do nothing once
@@ -1438,16 +1451,18 @@ sp_gram_kernel(const __grid_constant__ SsArgs a, const KoStepState* st) {
     });
 }
 
-// ---- the update as a device-driven graph -------------------------------------------------
+// ---- the update on the device -------------------------------------------------------------
 // kOmega::Solve (kOmega.cpp:31-73: the doubling test, then sub-steps of
-// assembly + both solves, halving dt on a NaN residual) as the body of one
-// WHILE node: assembly, residual, Gram and update sweep, each of which does
-// nothing where the state does not ask for it; a one-thread kernel at its end
-// takes every decision and sets the node's condition
-// (cudaGraphSetConditional), so that a time step needs no host round trip and
-// the usual step runs the body once.  The loop is bounded by counters: a solve
-// by its round cap, an update by the halving cap (steps_per_lb <= 2^20) and a
-// total of KU_MAX_SUBSTEPS solves.
+// assembly + both solves, halving dt on a NaN residual) as four launches:
+// assembly, Gram sweep, update sweep, and a cooperative kernel for whatever
+// the first three did not finish: cycles that asked for more powers, restarts,
+// sub-steps.  A usual step has nothing left, and that kernel returns at once;
+// so a time step needs neither a host round trip nor a conditional graph node
+// (a WHILE node around the same kernels cost 8 to 10 us a step, and a launch
+// for a residual sweep that has nothing to do 2).  The update sweep's last
+// block takes the decisions of a round; the loop is bounded by counters: a
+// solve by its round cap, an update by the halving cap (steps_per_lb <= 2^20)
+// and a total of KU_MAX_SUBSTEPS solves.
 
 constexpr int KU_MAX_SUBSTEPS = (1 << 21) + 64;  // above any sequence the halving cap allows
 
@@ -1462,6 +1477,7 @@ __global__ void ku_reset_kernel(KoStepState* st, double dt, int steps_per_lb) {
     st->launches = 0;
     st->fresh = 1;
     st->again = 0;
+    st->go = 0;
     st->updates = 0;
     st->launches_total = 0;
 }
@@ -1476,29 +1492,30 @@ __global__ void ku_fail_kernel(KoStepState* st, int n, int mask) {
 __host__ __device__ __forceinline__ bool ku_doubles(int time_since_change, int steps_per_lb) {
     return time_since_change + 1 >= 20 && steps_per_lb != 1;
 }
-// Time step of the assembly of the body about to run.
+// Time step of the assembly about to run.
 __device__ __forceinline__ double ku_dt(const KoStepState* st) {
     const double dt = ldc(&st->dt);
     return ldc(&st->fresh) && ku_doubles(ldc(&st->time_since_change), ldc(&st->steps_per_lb)) ? dt * 2.0 : dt;
 }
 
-// The assembly of a sub-step, and the control block of its solve (written by
-// the first block; the sweeps that read it are later launches).
+// The assembly of an update's first sub-step, and the control block of its
+// solve (written by the first block; the sweeps that read it are later
+// launches).
 template <typename FT>
 __global__ void __launch_bounds__(KM_WARPS * 32, KOFM_ASM_MINBLOCKS)
 ku_assemble_kernel(const AsmParams p, GmresControl* ctl, GridBarrier* bar, SsQueue* queue, KoStepState* st,
                    const int* lhint, int K) {
-    if (ldc(&st->status) || ldc(&st->again)) return;
+    if (ldc(&st->status)) return;
     if (blockIdx.x == 0)
-        ss_ctl_init(ctl, bar, queue, st, ss_hint_levels(__ldcg(lhint), K), ss_hint_levels(__ldcg(lhint + 1), K));
-    km_assemble<FT>(p, ku_dt(st));
+        ss_ctl_init<false>(ctl, bar, queue, st, ss_hint_levels(__ldcg(lhint), K), ss_hint_levels(__ldcg(lhint + 1), K));
+    km_assemble<FT>(p, ku_dt(st), blockIdx.x * KM_WARPS + (threadIdx.x >> 5));
 }
 
-constexpr int KU_BODY_LAUNCHES = 5;  // assembly, residual, Gram and update sweep, end
+constexpr int KU_LAUNCHES = 4;  // assembly, Gram and update sweep, the rest
 
-// Decisions at the end of a body (one thread): whether another one runs.
-__device__ __forceinline__ bool ku_body_end(GmresControl* ctl, KoStepState* st, int max_rounds) {
-    if (st->status) return false;
+// Decisions after `rounds` rounds of a solve (one thread): what is left of the
+// update.
+__device__ __forceinline__ void ku_round_end(GmresControl* ctl, KoStepState* st, int rounds, int max_rounds) {
     if (st->fresh) {
         if (ku_doubles(st->time_since_change, st->steps_per_lb)) {
             st->steps_per_lb /= 2;
@@ -1507,14 +1524,13 @@ __device__ __forceinline__ bool ku_body_end(GmresControl* ctl, KoStepState* st, 
         st->time_since_change = st->time_since_change + 1 >= 20 ? 0 : st->time_since_change + 1;
         st->cur = 0;
         st->substeps = 0;
-        st->launches = 0;
+        st->launches = KU_LAUNCHES;
+        st->launches_total += KU_LAUNCHES;
         st->updates++;
         st->fresh = 0;
     }
-    st->launches += KU_BODY_LAUNCHES;
-    st->launches_total += KU_BODY_LAUNCHES;
     st->again = 0;
-    const int r = ldc(&ctl->rounds) + 1;
+    const int r = ldc(&ctl->rounds) + rounds;
     __stcg(&ctl->rounds, r);
     bool go = false;
     if (ldc(&ctl->error)) {
@@ -1545,25 +1561,53 @@ __device__ __forceinline__ bool ku_body_end(GmresControl* ctl, KoStepState* st, 
         }
     }
     if (!go) st->fresh = 1;
-    return go;
+    st->go = go;
 }
 
 // The update sweep.
 template <typename FT>
 __global__ void __launch_bounds__(SS_BLOCK, 1)
-sp_update_kernel(const __grid_constant__ SsArgs a, const KoStepState* st) {
+sp_update_kernel(const __grid_constant__ SsArgs a, KoStepState* st, int max_rounds) {
     if (sp_stopped(st)) return;
     ss_specialise(a, [&] {
         if (ss_begin(a, false, ss_upd_levels(a, 0), ss_upd_levels(a, 1))) ss_upd_unit<FT>(a, blockIdx.x);
         ss_write_units<FT>(a);
-        if (sp_last_block(a) && threadIdx.x == 0) ss_upd_serial(a);
+        if (sp_last_block(a) && threadIdx.x == 0) {
+            ss_upd_serial(a);
+            if (st) ku_round_end(a.ctl, st, 1, max_rounds);
+        }
     });
 }
 
-// End of the body (its own kernel: a call of the device runtime in the update
-// sweep keeps the compiler from moving registers between its warpgroups).
-__global__ void ku_end_kernel(GmresControl* ctl, KoStepState* st, int max_rounds, cudaGraphConditionalHandle body) {
-    if (threadIdx.x == 0) cudaGraphSetConditional(body, ku_body_end(ctl, st, max_rounds) ? 1u : 0u);
+// What is left of an update (cooperative; returns at once where nothing is).
+template <typename FT>
+__global__ void __launch_bounds__(SS_BLOCK, 1)
+ku_rest_kernel(const __grid_constant__ SsArgs a, const __grid_constant__ AsmParams p, KoStepState* st, int max_rounds) {
+    if (sp_stopped(st) || !ldc(&st->go)) return;
+    ss_specialise(a, [&] {
+        // warps whose row rings of the assembly fit in the march's shared memory
+        constexpr int AW = (int)(SS_GRAM_DSMEM / km_ring_bytes<FT>()) < SS_WARPS ? (int)(SS_GRAM_DSMEM / km_ring_bytes<FT>())
+                                                                               : SS_WARPS;
+        while (true) {
+            if (!ldc(&st->again)) {
+                if (blockIdx.x == 0)
+                    ss_ctl_init<true>(a.ctl, a.bar, a.queue, st, ss_hint_levels(__ldcg(a.lhint), a.K),
+                                      ss_hint_levels(__ldcg(a.lhint + 1), a.K));
+                const int warp = threadIdx.x >> 5, warps = km_warps(p);
+                if (warp < AW)
+                    for (int w = blockIdx.x * AW + warp; w < warps; w += gridDim.x * AW) km_assemble<FT>(p, ku_dt(st), w);
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                if (!ss_sync(a, [] {})) break;
+            }
+            const int rounds = ss_solve<FT>(a);
+            if (!ss_sync(a, [&] { if (threadIdx.x == 0) ku_round_end(a.ctl, st, rounds, max_rounds); })) break;
+            if (!ldc(&st->go)) return;
+        }
+        if (threadIdx.x == 0) {  // a barrier's wait ran out
+            st->status = KOFM_ERR_TIMEOUT;
+            st->go = 0;
+        }
+    });
 }
 
 }  // namespace kofm

@@ -67,3 +67,46 @@ def test_solved_fields_satisfy_the_rows(kofm_lib, form, nx, ny, krylov):
                 bound = 1.01 * REL_TOL * np.linalg.norm(rhs) + 2.5 * np.finfo(float).eps * np.linalg.norm(x1)
                 assert np.abs(coef).sum(0).max() < 1.5
                 assert np.linalg.norm(r) <= bound, (np.linalg.norm(r), bound)
+
+
+@pytest.mark.parametrize("krylov,storage", [(2, _abi.STORE_FP64), (10, _abi.STORE_FP64), (3, _abi.STORE_FP32)])
+def test_restarts_and_substeps_finish_on_the_device(kofm_lib, krylov, storage):
+    """Restarts, and the sub-steps after a NaN residual, of the update that is
+    enqueued without a host round trip: the fields of the host-driven rounds.
+    Each solve's residual is at most REL_TOL ||b'||, which with off-diagonal row
+    sums of at most q < 1 moves d by REL_TOL ||b'|| / (1 - q) at any node; four
+    solves (the last two of the sub-steps), and a factor 2 for what a difference
+    adds to the next rows.  FP32 fields add a rounding a solve."""
+    nx, ny = 301, 43
+    ch = G.straight_channel(nx, ny)
+    f = perturbed_state(ch, seed=3, u_mean=0.05, rho_amp=1e-4, u_amp=5e-3, neq_amp=1e-5)
+    k, o, nut, s = komega_state(ch, seed=4)
+    got = []
+    for form in (0, 3):
+        d = desc_default()
+        d.nx, d.nx_full, d.ny = nx, nx, ny
+        d.tau, d.fterm, d.mu = 1.0 / (3 * 1e-3 + 0.5), 1e-7, 1e-3
+        d.use_komega, d.storage = 1, storage
+        d.komega_rel_tol, d.komega_abs_tol = REL_TOL, 0.0
+        d.krylov_dim, d.komega_classic = krylov, form
+        d.komega_max_iters = 10000
+        with Lattice(d) as L:
+            L.set_geometry(ch.ntype, ch.wallD, ch.dX)
+            L.set_state(f, k, o, nut, s)
+            L.step(2)
+            _, K, O, _, _ = L.get_state()
+            st = L.stats()
+            assert max(st.omega_restarts, st.k_restarts) > 2  # more than the first cycle
+            L.debug_fail_solves(1, mask=1)  # the next solve reports a NaN residual: two sub-steps
+            L.step(1)
+            st = L.stats()
+            assert st.steps_per_lb == 2
+            _, K2, O2, _, _ = L.get_state()
+            rows = [L.komega_rows(i) for i in (1, 0)]
+            got.append((K, O, K2, O2))
+    eps = np.finfo(np.float32 if storage == _abi.STORE_FP32 else np.float64).eps
+    for i, (a, b) in enumerate(zip(*got)):
+        coef, rhs = rows[i % 2]
+        q = np.abs(coef.reshape(4, -1)).sum(0).max()
+        bound = 4 * 2 * 2 * REL_TOL * np.linalg.norm(rhs) / (1 - q) + 4 * eps * np.abs(a).max()
+        assert q < 1 and np.abs(a - b).max() <= bound, (i, q, np.abs(a - b).max(), bound)
