@@ -611,9 +611,13 @@ cudaError_t launch_lb(kofm_ctx* c, const LbParams& p, bool komega, bool phase0) 
     if (komega) {
         if (phase0) lb_step_kernel<ST, AT, true, true, NEQ, FT, ROW><<<grid, block, 0, c->stream>>>(p);
         else lb_step_kernel<ST, AT, true, false, NEQ, FT, ROW><<<grid, block, 0, c->stream>>>(p);
-    } else {
+    } else if (NEQ) {  // (its read-only loads of the last step's moments may not move above a wait)
         if (phase0) lb_step_kernel<ST, AT, false, true, NEQ, FT, ROW><<<grid, block, 0, c->stream>>>(p);
         else lb_step_kernel<ST, AT, false, false, NEQ, FT, ROW><<<grid, block, 0, c->stream>>>(p);
+    } else {
+        return launch_after(phase0 ? lb_step_kernel<ST, AT, false, true, NEQ, FT, ROW>
+                                   : lb_step_kernel<ST, AT, false, false, NEQ, FT, ROW>,
+                            grid, block, c->stream, p);
     }
     return cudaGetLastError();
 }

@@ -503,7 +503,11 @@ __device__ __forceinline__ void lb_block(const LbParams& p, int bx, int by, int 
 
 template <typename ST, typename AT, bool KOMEGA, bool PHASE0, bool NEQ = false, typename FT = float, bool ROW = false>
 __global__ void __launch_bounds__(128, ((NEQ && sizeof(AT) == 8) || sizeof(FT) == 8) ? 1 : KOFM_LB_MINBLOCKS)
-lb_step_kernel(const LbParams p) {
+lb_step_kernel(const LbParams in) {
+    if constexpr (!KOMEGA && !NEQ) grid_wait();
+    // A copy: the parameters are fetched into registers at once (and, with
+    // grid_wait, while the kernel waits) instead of where each is used.
+    LbParams p = in;
     lb_block<ST, AT, KOMEGA, PHASE0, NEQ, FT, ROW>(p, blockIdx.x, blockIdx.y, gridDim.x);
 }
 
