@@ -110,15 +110,15 @@ def open_lattices(workloads, storage=_abi.STORE_FP16_NEQ, caps=None):
 
 def solver_caps(workloads, policy, sms: int):
     """Per-lattice caps on the solver grid for one tuning policy:
-    "auto" -- none (each solver may take two blocks per SM);
-    "share" -- two blocks per SM split over the k-omega lattices in proportion
-    to their node counts (at least 8 each), so concurrent solvers fit side by
-    side; an integer -- that cap for every lattice."""
+    "auto" -- none (each solver may take one block per SM);
+    "share" -- the SMs split over the k-omega lattices in proportion to their
+    node counts (a block of the solver takes a whole SM), so concurrent solvers
+    fit side by side; an integer -- that cap for every lattice."""
     if policy == "auto":
         return [0] * len(workloads)
     if policy == "share":
         tot = sum(w.nodes for w in workloads if w.komega) or 1
-        return [max(8, int(2 * sms * w.nodes / tot)) if w.komega else 0 for w in workloads]
+        return [max(1, int(sms * w.nodes / tot)) if w.komega else 0 for w in workloads]
     return [int(policy)] * len(workloads)
 
 
