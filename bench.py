@@ -162,7 +162,7 @@ def replica_value(nodes: int, steps: int, world: int, ms: float) -> float:
 # bytes (traffic grows with the nodes and the sweeps of a launch).
 SOLVER_TRAFFIC_RATIO = {
     "gmres_kernel": 4.7967e9 / (1076 * 4194304),   # one vector per sweep
-    "sstep_kernel": None,                          # one sweep per cycle's powers
+    "sstep_kernel": None,                          # two sweeps per cycle
     "sstep_phases": None,                          # the same, one launch per sweep
 }
 
@@ -466,7 +466,7 @@ def main():
     ap.add_argument("--workload", default="komega_straight_16384x1024")
     ap.add_argument("--storage", default="fp32", choices=["fp32", "fp16", "bf16", "fp16neq", "fp16neq32", "fp16row", "fp64"])
     ap.add_argument("--solver", default="sstep", choices=["sstep", "sstep_host", "sstep_coop", "classic"],
-                    help="k-omega solve: a cycle's Krylov directions in one sweep, each sweep "
+                    help="k-omega solve: two marching sweeps per cycle, each sweep "
                          "its own launch in a device-driven update graph (default) or enqueued "
                          "round by round by the host (sstep_host), or all in one cooperative "
                          "launch (sstep_coop); or one vector per sweep (classic)")

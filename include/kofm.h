@@ -145,12 +145,12 @@ typedef struct kofm_desc {
     double t_in;              /* TFD_X_IN_VAL (TFD_X_IN 2.0): inlet temperature
                                  and upper clamp of T in the source term */
     int32_t thermal_max_iters;/* THERMAL_MAX_ITERS (1000) */
-    int32_t komega_classic;   /* k-omega solver form: 0 (default) builds all
-                                 Krylov directions of a cycle in one sweep
-                                 (powers of the off-diagonal operator, Gram
-                                 matrix, the simpler-GMRES steps in that
-                                 basis), each sweep its own kernel launch and
-                                 the host enqueueing one round at a time;
+    int32_t komega_classic;   /* k-omega solver form: 0 (default) takes two
+                                 sweeps per cycle (powers of the off-diagonal
+                                 operator and their Gram matrix, the simpler-
+                                 GMRES steps in that basis, the powers again
+                                 for the update), each its own kernel launch
+                                 and every decision taken on the device;
                                  2 is the same solve in one cooperative
                                  launch (the form kofm_batch graphs capture);
                                  3 is form 0 with the host enqueueing each
@@ -194,7 +194,7 @@ typedef struct kofm_stats {
     double solver_bytes_per_node;       /* algorithmic HBM bytes per lattice node of the
                                            last k-omega solve (both systems): every
                                            array its sweeps stream, counted once per sweep */
-    int32_t omega_powers, k_powers;     /* one-sweep cycles: powers computed (all rounds) */
+    int32_t omega_powers, k_powers;     /* two-sweep cycles: powers of the Gram sweeps (all rounds) */
     int32_t solver_launches;            /* kernel launches of the last k-omega solve */
     int32_t solver_rounds;              /* rounds of the last solve (phase launches:
                                            powers + Gram + update sweeps; 1 otherwise) */
@@ -469,8 +469,8 @@ void* kofm_stream(kofm_ctx* ctx);
  * lattice rows x 128 columns of one lattice; kofm_batch_create_tiled chooses
  * tile_rows, 0 or kofm_batch_create: 2; -1 keeps one collide launch per
  * lattice in the lattice's own branch); then every k-omega lattice's
- * assembly and solve run as concurrent graph branches (the one-sweep-per-
- * cycle solver in its one-launch form, komega_classic 2, for contexts of the
+ * assembly and solve run as concurrent graph branches (the two-sweep
+ * solver in its one-launch form, komega_classic 2, for contexts of the
  * phase-launch forms).  Requirements checked by kofm_batch_create: all
  * contexts on one device, each past its first step (kofm_step /
  * kofm_lb_step called at least once), and for k-omega lattices

@@ -32,11 +32,11 @@ __device__ __forceinline__ void after_wait(P& p) {
 }
 
 // Launch of a kernel that begins with grid_wait().  For chains of short kernels,
-// where the gap between two of them counts: 2000 laminar steps of 256x64 took
-// 6.15 us each and take 3.7, of 1999x501 with curved walls 30.7 and 25.1.  Not
-// for the kernels of a turbulent step: the collide, placed while the update's
-// end still runs, took 413 -> 426 us a step at 4096x512 and 2711 -> 2742 at
-// 16384x1024, and gained nothing at 256x64.
+// where the gap between two of them counts: a laminar step of 256x64 took 6.15
+// us and takes 3.8 (4.76 without the collide's early fetch of its parameters),
+// of 31x17 6.2 and 3.8.  Not for the kernels of a turbulent step: the collide,
+// placed while the update's end still runs, took 413 -> 426 us a step at
+// 4096x512 and 2711 -> 2742 at 16384x1024, and gained nothing at 256x64.
 template <typename... P, typename... A>
 inline cudaError_t launch_after(void (*fn)(P...), dim3 grid, dim3 block, cudaStream_t stream, A... args) {
     cudaLaunchAttribute at[1];

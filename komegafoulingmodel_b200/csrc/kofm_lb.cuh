@@ -506,7 +506,9 @@ __global__ void __launch_bounds__(128, ((NEQ && sizeof(AT) == 8) || sizeof(FT) =
 lb_step_kernel(const LbParams in) {
     if constexpr (!KOMEGA && !NEQ) grid_wait();
     // A copy: the parameters are fetched into registers at once (and, with
-    // grid_wait, while the kernel waits) instead of where each is used.
+    // grid_wait, while the kernel waits) instead of where each is used.  The
+    // kernel alone, us, before and after: 16384x1024 turbulent 551 and 499,
+    // laminar 373 and 308, FP16 against its moments 8192x512 302 and 256.
     LbParams p = in;
     lb_block<ST, AT, KOMEGA, PHASE0, NEQ, FT, ROW>(p, blockIdx.x, blockIdx.y, gridDim.x);
 }

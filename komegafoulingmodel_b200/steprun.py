@@ -7,8 +7,7 @@ k-omega step run.
 
 --form is kofm_desc.komega_classic: 0 the device-driven update graph
 (default), 1 one Krylov vector per sweep, 2 the one-launch solve, 3 the
-phase kernels with the host enqueueing each round (the kernels of form 0;
-ncu lists kernels that conditional graph nodes launch only in this form).
+phase kernels with the host enqueueing each round (the kernels of form 0).
 """
 from __future__ import annotations
 
