@@ -117,6 +117,7 @@ struct kofm_ctx {
     int ss_blocks = 0, ss_maxu = 0, sp_gram_blocks = 0, sp_upd_blocks = 0, sp_resid_blocks = 0;
     short ss_gram_rows[SS_MAXL + 2][SS_MAXL + 2] = {}, ss_upd_rows[SS_MAXL + 2][SS_MAXL + 2] = {};
     int ss_hint[2] = {0, 0};          // host copy of ss_lhint (first-round powers)
+    bool first_solve = false;         // the next solve is a loaded state's first (sp_first_gram_kernel)
     // the k-omega update as a device-driven CUDA graph (kofm_stepgraph.inc)
     KoStepState* kst = nullptr;       // sub-stepping state (device)
     KoStepState* h_kst = nullptr;     // pinned copy
@@ -796,9 +797,9 @@ int kofm_create(const kofm_desc* d, kofm_ctx** out) {
         ALLOC_FIELD(c->S, 3 * D);
         ALLOC_FIELD(c->nut, D);
         // (the form the entry points take: solver_form)
-        const bool basis = d->komega_full_cycle || d->komega_classic == 1;
+        const bool classic = d->komega_full_cycle || d->komega_classic == 1;
         int s2 = ko_solver_alloc(c->sys, &c->ctl, &c->gpart, &c->bar, &c->solver_blocks,
-                                 c->P, d->ny, d->krylov_dim, c->dev, d->solver_max_blocks, basis);
+                                 c->P, d->ny, d->krylov_dim, c->dev, d->solver_max_blocks, classic);
         if (!s2) s2 = ss_solver_alloc(c);
         if (s2) { kofm_destroy(c); return s2; }
         if (cudaMallocHost(&c->h_ctl, sizeof(GmresControl)) != cudaSuccess ||
@@ -1042,6 +1043,7 @@ int kofm_set_state(kofm_ctx* c, const double* f, const double* k, const double* 
     if (d.use_komega) {
         ug_pull(c);  // updates still in flight finish first
         ug_reset(c);
+        c->first_solve = true;
         c->launches_host = 0;
         c->stats.solver_launches_total = 0;
     }

@@ -47,7 +47,8 @@ struct KoSystem {
     double* r = nullptr;      // [D] residual of restarts >= 1
     double* x = nullptr;     // [D] correction
     double* V = nullptr;      // [K x D] Krylov basis (orthogonalised, unscaled; interleaved) of the
-                              // one-vector-per-sweep form; the other forms keep no basis
+                              // one-vector-per-sweep form; the powers p_1 .. p_K of a loaded
+                              // state's first solve in the others (null where memory is short)
 };
 
 struct AsmParams {

@@ -30,8 +30,11 @@
 // fired by then is run again with the powers up to the Krylov dimension.
 // In FP64 the truncation tests see rounding of the size the reference's own
 // classical Gram-Schmidt has (both lose orthogonality like eps cond^2), so the
-// cut of a converged cycle moves by a vector or two while restart counts and
-// the solution agree to far below the tolerance.
+// cut of a converged cycle moves by a vector or two with the order of a sum, and
+// with it the end residual, between about 1e-6 and 1e-9 ||b'|| (the tolerance is
+// 1e-4).  In a running channel that is far below the fields' rounding; in the
+// first solve of a loaded state it need not be, so that one takes its sums in a
+// fixed order (sp_first_gram_kernel).
 #pragma once
 #include "kofm_gmres.cuh"
 
@@ -152,11 +155,16 @@ __device__ __forceinline__ void ss_rank(SsCycleSmem& cs, int n) {
 // shift, one product with G, two sums over the lanes and a square root per
 // vector.  The warp's halves do the same work, so that every lane holds what
 // the tests read.
+// ORDERED: with the estimator, the quotients and the order of the sums as the
+// reference's formulas have them (GMRESSolver.cpp:300-330), for sums whose
+// rounding decides the result (sp_first_gram_kernel); in every solve that would
+// be 3 us of a step's 57 at 256x64.
 struct SsCycle {
     double V[SS_MAXL];  // this lane's coefficient of v_0 .. v_{built-1}
     int built;          // vectors built
     int cut;            // 0: none (all L vectors passed), 1: diag(R), 2: xi, 3: all K built
 };
+template <bool ORDERED>
 __device__ __forceinline__ void ss_cycle(SsCycle& c, SsCycleSmem& cs, int L, int K, double rel_tol, double rinv) {
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 15;
@@ -178,21 +186,27 @@ __device__ __forceinline__ void ss_cycle(SsCycle& c, SsCycleSmem& cs, int L, int
 #pragma unroll
         for (int j = 0; j <= SS_MAXL; ++j) {
             const double wj = __shfl_sync(FULL, w, j);
-            if (j & 1) a1 += g[j] * wj;
-            else a0 += g[j] * wj;
+            if (!ORDERED && (j & 1)) a1 += g[j] * wj;
+            else if (j < n) a0 += g[j] * wj;
         }
         double Gw = a0 + a1;
         double h[SS_MAXL];
 #pragma unroll
-        for (int j = 0; j < k; ++j) h[j] = ss_sum16(w * GV[j]);
+        for (int j = 0; j < k; ++j) h[j] = ss_sum16(ORDERED ? __dmul_rn(w, GV[j]) : w * GV[j]);
 #pragma unroll
         for (int j = 0; j < k; ++j) {
             w -= h[j] * c.V[j];
             Gw -= h[j] * GV[j];
         }
-        const double nk2 = ss_sum16(w * Gw);
-        const double inv = nk2 > 0.0 ? rsqrt(nk2) : 0.0;  // a vanishing direction cuts (diag test)
-        const double nk = nk2 > 0.0 ? nk2 * inv : 0.0;
+        const double nk2 = ss_sum16(ORDERED ? __dmul_rn(w, Gw) : w * Gw);
+        double inv, nk;  // a vanishing direction cuts (diag test)
+        if (ORDERED) {
+            nk = nk2 > 0.0 ? sqrt(nk2) : 0.0;
+            inv = nk > 0.0 ? 1.0 / nk : 0.0;
+        } else {
+            inv = nk2 > 0.0 ? rsqrt(nk2) : 0.0;
+            nk = nk2 > 0.0 ? nk2 * inv : 0.0;
+        }
         c.V[k] = w * inv;
         GV[k] = Gw * inv;
         const double xi = rinv * __shfl_sync(FULL, GV[k], 0, 16);  // <r / rho0, v_k>
@@ -209,7 +223,7 @@ __device__ __forceinline__ void ss_cycle(SsCycle& c, SsCycleSmem& cs, int L, int
         if (nk < rel_tol * r00) c.cut = 1;
         else if (x >= rho) c.cut = 2;
         else {
-            rho = sqrt((rho - x) * (rho + x));  // rho sin(acos(xi / rho))
+            rho = ORDERED ? rho * sin(acos(xi / rho)) : sqrt((rho - x) * (rho + x));
             if (k == K - 1) c.cut = 3;
         }
     }
@@ -1063,48 +1077,55 @@ __device__ __forceinline__ void ss_gram_unit(const SsArgs& a, int n) {
     }
 }
 
-// Serial step of the Gram sweep, run by the last block: the sums over the
-// units in a fixed order, then per system one warp for the cycle and one for
-// the basis's rank.
-__device__ __forceinline__ void ss_gram_serial(const SsArgs& a) {
-    const SsPlan& pl = ss_sm().plan;
+// Serial step of a Gram sweep of lev[s] levels (-1: none), run by the last
+// block: sums(tot) gets the entries, then per system one warp for the cycle and
+// one for the basis's rank.  bytes: what the sweep moved, per node.
+template <bool ORDERED, typename F>
+__device__ __forceinline__ void ss_gram_serial(const SsArgs& a, const int (&lev)[2], const double (&bytes)[2], F sums) {
     __shared__ double tot[2][SS_NG];
     __shared__ GmresSys sS[2];
     __shared__ SsCycleSmem cs[2];
     const int warp = threadIdx.x >> 5;
     SsSysWord w[2];
-    int ng[2], n[2];
 #pragma unroll
-    for (int s = 0; s < 2; ++s) {
-        w[s].load(a.ctl, s);
-        ng[s] = pl.lev[s] > 0 ? (pl.lev[s] + 1) * (pl.lev[s] + 2) / 2 : 0;
-        n[s] = ng[s] ? pl.strips[s] * pl.rows : 0;
-    }
-    ss_unit_sums(a, ng, n, tot);
+    for (int s = 0; s < 2; ++s) w[s].load(a.ctl, s);
+    sums(tot);
     for (int s = 0; s < 2; ++s) w[s].put(sS[s]);
     ss_sync_march();
-    const int s = warp & 1, L = pl.lev[s];
+    const int s = warp & 1, L = lev[s];
     if (L > 0) {
-        if (threadIdx.x == 32 * s)  // p_0 and the coefficients of the sweep, per node
-            sS[s].abytes += 40.0 * pl.parts[s];
+        if (threadIdx.x == 32 * s) sS[s].abytes += bytes[s];
         ss_gram_begin(a, sS[s], tot[s], L, cs[s]);
     }
     ss_sync_march();
     SsCycle c;
     if (L > 0 && sS[s].active) {
-        if (warp < 2) ss_cycle(c, cs[s], L, a.K, a.rel_tol, sS[s].rinv);
+        if (warp < 2) ss_cycle<ORDERED>(c, cs[s], L, a.K, a.rel_tol, sS[s].rinv);
         else if (warp < 4) ss_rank(cs[s], L + 1);
     }
     ss_sync_march();
     if (warp < 2 && L > 0 && sS[s].active) ss_gram_end(a, sS[s], s, L, cs[s], c);
     ss_sync_march();
     for (int q = 0; q < 2; ++q)
-        if (pl.lev[q] > 0) sp_sys_store(a.ctl, q, sS[q]);
+        if (lev[q] > 0) sp_sys_store(a.ctl, q, sS[q]);
     if (threadIdx.x == 0) {
         trace_barrier(a.ctl);
         __stcg(&a.ctl->passes, ldc(&a.ctl->passes) + 1);
         __stcg(&a.ctl->any_active, (int)(sS[0].active || sS[1].active));
     }
+}
+// After a march: the sums over the units in a fixed order.
+__device__ __forceinline__ void ss_gram_serial(const SsArgs& a) {
+    const SsPlan& pl = ss_sm().plan;
+    int ng[2], n[2];
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+        ng[s] = pl.lev[s] > 0 ? (pl.lev[s] + 1) * (pl.lev[s] + 2) / 2 : 0;
+        n[s] = ng[s] ? pl.strips[s] * pl.rows : 0;
+    }
+    // p_0 and the coefficients
+    ss_gram_serial<false>(a, pl.lev, {40.0 * pl.parts[0], 40.0 * pl.parts[1]},
+                          [&](double (*tot)[SS_NG]) { ss_unit_sums(a, ng, n, tot); });
 }
 
 // Levels of the update sweep of system s (-1: nothing for a march to do).
@@ -1448,6 +1469,110 @@ sp_gram_kernel(const __grid_constant__ SsArgs a, const KoStepState* st) {
         if (!ss_begin(a, true, ss_gram_levels(a, 0), ss_gram_levels(a, 1))) return;
         ss_gram_unit(a, blockIdx.x);
         if (sp_last_block(a)) ss_gram_serial(a);
+    });
+}
+
+// ---- the first Gram sums of a loaded state ------------------------------------------------
+// What ends a cycle is rounding (in exact arithmetic |xi_k| stays below rho): a
+// last digit of a Gram sum decides whether it ends a vector sooner, at a residual
+// of about 1e-6 or of 1e-9 ||b'||.  In a running channel neither shows.  In the
+// first solve after kofm_set_state it can: beside a curved wall that passes a
+// node at 1e-4, omega starts at 6 nu / (0.075 d^2) and is 1000 at most afterwards,
+// ||b'|| is 1e5 to 1e7, and 1e-6 of it is percents of the omega a node further,
+// which later steps do not take back.  So that solve takes its sums in one fixed
+// order, whatever the form, the row ranges and the units of a march: the nodes in
+// so_ranges(L) ranges of whole 32-column groups, a thread every 256th node of a
+// range, then the threads of a warp, the warps, the ranges; and its cycle takes
+// the reference's formulas to the letter (ss_cycle<true>).  Measured on 242
+// channels with wavy walls, the fields after 6 steps: with the marches' sums 17
+// differ by over 0.8% of omega or k at a node from the fixed order's, by up to
+// 60%; here the three forms agree to 2e-7.
+//
+// The powers are formed one after the other in memory and summed in a pass of
+// their own: a loaded state's first step takes 80 us more at 256x64, 350 at
+// 4096x512 and 2600 at 16384x1024.  Where the memory for the powers could not be
+// had, the first solve marches like the others.
+__host__ __device__ constexpr int so_ranges(int L) { return 148 * (L >= 9 ? 1 : L >= 6 || L == 1 ? 2 : 3); }
+constexpr int SO_MAX_RANGES = 148 * 3;
+
+// p_{j+1} = N p_j of both systems.
+__global__ void __launch_bounds__(SS_THREADS) sp_power_kernel(const __grid_constant__ SsArgs a, const KoStepState* st, int j) {
+    if (sp_stopped(st)) return;
+    const int x = blockIdx.x * SS_THREADS + threadIdx.x;
+    if (x >= a.nx) return;
+    const int xw = x > 0 ? x - 1 : a.nx - 1, xe = x + 1 < a.nx ? x + 1 : 0;
+    const KoSystem& S = a.sys[blockIdx.z];
+    const double* p = j == 0 ? S.rhs : S.V + (j - 1) * a.D;
+    double* out = S.V + j * a.D;
+    for (int y = blockIdx.y; y < a.ny; y += gridDim.y) {
+        const long long row = (long long)y * a.P, g = row + x;
+        const double* cf = S.coef + ilv(4, 0, g);
+        // rows 0 and ny - 1 are solid: their off-diagonals are 0
+        const double pS = y > 0 ? p[g - a.P] : 0.0, pN = y + 1 < a.ny ? p[g + a.P] : 0.0;
+        // (the roundings are part of the result here, so they are written out)
+        out[g] = __fma_rn(cf[64], pN, __fma_rn(cf[0], p[row + xe], __fma_rn(cf[96], pS, __dmul_rn(cf[32], p[row + xw]))));
+    }
+}
+
+// The sums of a range and, in the last block, the serial step; in place of the
+// Gram sweep.  Block b: range b of omega, then of k.
+__global__ void __launch_bounds__(SS_THREADS, 1)
+sp_first_gram_kernel(const __grid_constant__ SsArgs a, const KoStepState* st) {
+    __shared__ double red[SS_WARPS][SS_NG];
+    if (sp_stopped(st)) return;
+    const int lev[2] = {ss_gram_levels(a, 0), ss_gram_levels(a, 1)};
+    if (lev[0] < 0 && lev[1] < 0) return;
+    // [slot][range] of each system
+    double* const part[2] = {a.part, a.part + (long long)SS_NG * SO_MAX_RANGES};
+    const int sys = blockIdx.x >= SO_MAX_RANGES, r = blockIdx.x - sys * SO_MAX_RANGES, L = lev[sys];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (L > 0 && r < so_ranges(L)) {
+        const int ranges = so_ranges(L);
+        const double* const p0 = a.sys[sys].rhs;
+        const double* const V = a.sys[sys].V;
+        const long long n32 = a.D / 32, g1 = n32 * (r + 1) / ranges * 32;
+        double s[SS_NG], p[SS_MAXL + 1];
+#pragma unroll
+        for (int i = 0; i < SS_NG; ++i) s[i] = 0.0;
+        auto load = [&](long long g) {
+#pragma unroll
+            for (int j = 0; j <= SS_MAXL; ++j) p[j] = j <= L && g < g1 ? __ldcg(j == 0 ? p0 + g : V + (j - 1) * a.D + g) : 0.0;
+        };
+        long long g = n32 * r / ranges * 32 + threadIdx.x;
+        load(g);
+        for (; g < g1; g += SS_THREADS) {
+            double q[SS_MAXL + 1];
+#pragma unroll
+            for (int j = 0; j <= SS_MAXL; ++j) q[j] = p[j];
+            load(g + SS_THREADS);
+#pragma unroll
+            for (int j = 0; j <= SS_MAXL; ++j)
+#pragma unroll
+                for (int i = 0; i <= j; ++i) s[ss_gslot(i, j)] = __fma_rn(q[i], q[j], s[ss_gslot(i, j)]);
+        }
+#pragma unroll
+        for (int i = 0; i < SS_NG; ++i) {
+            double x = s[i];
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1) x += __shfl_down_sync(0xffffffffu, x, off);
+            if (lane == 0) red[warp][i] = x;
+        }
+        ss_sync_march();
+        for (int i = threadIdx.x; i < SS_NG; i += SS_THREADS) {
+            double x = 0.0;
+#pragma unroll
+            for (int w = 0; w < SS_WARPS; ++w) x += red[w][i];
+            __stcg(part[sys] + (long long)i * ranges + r, x);
+        }
+    }
+    if (!sp_last_block(a)) return;
+    // a power: one and four coefficients in, one out; the sums: all in
+    ss_gram_serial<true>(a, lev, {56.0 * lev[0] + 8.0, 56.0 * lev[1] + 8.0}, [&](double (*tot)[SS_NG]) {
+        for (int s = 0; s < 2; ++s)
+            for (int i = warp; lev[s] > 0 && i < (lev[s] + 1) * (lev[s] + 2) / 2; i += SS_WARPS) {
+                const double v = sum_slot_warp(part[s], so_ranges(lev[s]), i);
+                if (lane == 0) tot[s][i] = v;
+            }
     });
 }
 
