@@ -29,6 +29,7 @@ int th_solver_alloc(kofm_ctx* c);
 int ko_solver_alloc(KoSystem* sys, GmresControl** ctl, double** part, unsigned int** bar,
                     int* nblocks, int P, int ny, int K, int dev, int max_blocks, bool basis);
 int ss_solver_alloc(kofm_ctx* c);
+void first_solve_alloc(kofm_ctx* c);
 void ko_system_free(KoSystem* s);
 static int ug_pull(kofm_ctx* c);
 static void ug_reset(kofm_ctx* c);
@@ -797,9 +798,9 @@ int kofm_create(const kofm_desc* d, kofm_ctx** out) {
         ALLOC_FIELD(c->S, 3 * D);
         ALLOC_FIELD(c->nut, D);
         // (the form the entry points take: solver_form)
-        const bool classic = d->komega_full_cycle || d->komega_classic == 1;
+        const bool basis = d->komega_full_cycle || d->komega_classic == 1;
         int s2 = ko_solver_alloc(c->sys, &c->ctl, &c->gpart, &c->bar, &c->solver_blocks,
-                                 c->P, d->ny, d->krylov_dim, c->dev, d->solver_max_blocks, classic);
+                                 c->P, d->ny, d->krylov_dim, c->dev, d->solver_max_blocks, basis);
         if (!s2) s2 = ss_solver_alloc(c);
         if (s2) { kofm_destroy(c); return s2; }
         if (cudaMallocHost(&c->h_ctl, sizeof(GmresControl)) != cudaSuccess ||
@@ -1044,6 +1045,7 @@ int kofm_set_state(kofm_ctx* c, const double* f, const double* k, const double* 
         ug_pull(c);  // updates still in flight finish first
         ug_reset(c);
         c->first_solve = true;
+        first_solve_alloc(c);
         c->launches_host = 0;
         c->stats.solver_launches_total = 0;
     }

@@ -187,7 +187,7 @@ __device__ __forceinline__ void ss_cycle(SsCycle& c, SsCycleSmem& cs, int L, int
         for (int j = 0; j <= SS_MAXL; ++j) {
             const double wj = __shfl_sync(FULL, w, j);
             if (!ORDERED && (j & 1)) a1 += g[j] * wj;
-            else if (j < n) a0 += g[j] * wj;
+            else if (!ORDERED || j < n) a0 += g[j] * wj;
         }
         double Gw = a0 + a1;
         double h[SS_MAXL];
@@ -1077,11 +1077,11 @@ __device__ __forceinline__ void ss_gram_unit(const SsArgs& a, int n) {
     }
 }
 
-// Serial step of a Gram sweep of lev[s] levels (-1: none), run by the last
+// Serial step of a Gram sweep of lev(s) levels (-1: none), run by the last
 // block: sums(tot) gets the entries, then per system one warp for the cycle and
-// one for the basis's rank.  bytes: what the sweep moved, per node.
-template <bool ORDERED, typename F>
-__device__ __forceinline__ void ss_gram_serial(const SsArgs& a, const int (&lev)[2], const double (&bytes)[2], F sums) {
+// one for the basis's rank.  bytes(s): what the sweep moved, per node.
+template <bool ORDERED, typename LEV, typename BYTES, typename SUMS>
+__device__ __forceinline__ void ss_gram_serial(const SsArgs& a, LEV lev, BYTES bytes, SUMS sums) {
     __shared__ double tot[2][SS_NG];
     __shared__ GmresSys sS[2];
     __shared__ SsCycleSmem cs[2];
@@ -1092,9 +1092,9 @@ __device__ __forceinline__ void ss_gram_serial(const SsArgs& a, const int (&lev)
     sums(tot);
     for (int s = 0; s < 2; ++s) w[s].put(sS[s]);
     ss_sync_march();
-    const int s = warp & 1, L = lev[s];
+    const int s = warp & 1, L = lev(s);
     if (L > 0) {
-        if (threadIdx.x == 32 * s) sS[s].abytes += bytes[s];
+        if (threadIdx.x == 32 * s) sS[s].abytes += bytes(s);
         ss_gram_begin(a, sS[s], tot[s], L, cs[s]);
     }
     ss_sync_march();
@@ -1107,7 +1107,7 @@ __device__ __forceinline__ void ss_gram_serial(const SsArgs& a, const int (&lev)
     if (warp < 2 && L > 0 && sS[s].active) ss_gram_end(a, sS[s], s, L, cs[s], c);
     ss_sync_march();
     for (int q = 0; q < 2; ++q)
-        if (lev[q] > 0) sp_sys_store(a.ctl, q, sS[q]);
+        if (lev(q) > 0) sp_sys_store(a.ctl, q, sS[q]);
     if (threadIdx.x == 0) {
         trace_barrier(a.ctl);
         __stcg(&a.ctl->passes, ldc(&a.ctl->passes) + 1);
@@ -1117,15 +1117,18 @@ __device__ __forceinline__ void ss_gram_serial(const SsArgs& a, const int (&lev)
 // After a march: the sums over the units in a fixed order.
 __device__ __forceinline__ void ss_gram_serial(const SsArgs& a) {
     const SsPlan& pl = ss_sm().plan;
-    int ng[2], n[2];
+    ss_gram_serial<false>(
+        a, [&](int s) { return pl.lev[s]; },
+        [&](int s) { return 40.0 * pl.parts[s]; },  // p_0 and the coefficients
+        [&](double (*tot)[SS_NG]) {
+            int ng[2], n[2];
 #pragma unroll
-    for (int s = 0; s < 2; ++s) {
-        ng[s] = pl.lev[s] > 0 ? (pl.lev[s] + 1) * (pl.lev[s] + 2) / 2 : 0;
-        n[s] = ng[s] ? pl.strips[s] * pl.rows : 0;
-    }
-    // p_0 and the coefficients
-    ss_gram_serial<false>(a, pl.lev, {40.0 * pl.parts[0], 40.0 * pl.parts[1]},
-                          [&](double (*tot)[SS_NG]) { ss_unit_sums(a, ng, n, tot); });
+            for (int s = 0; s < 2; ++s) {
+                ng[s] = pl.lev[s] > 0 ? (pl.lev[s] + 1) * (pl.lev[s] + 2) / 2 : 0;
+                n[s] = ng[s] ? pl.strips[s] * pl.rows : 0;
+            }
+            ss_unit_sums(a, ng, n, tot);
+        });
 }
 
 // Levels of the update sweep of system s (-1: nothing for a march to do).
@@ -1490,8 +1493,8 @@ sp_gram_kernel(const __grid_constant__ SsArgs a, const KoStepState* st) {
 //
 // The powers are formed one after the other in memory and summed in a pass of
 // their own: a loaded state's first step takes 80 us more at 256x64, 350 at
-// 4096x512 and 2600 at 16384x1024.  Where the memory for the powers could not be
-// had, the first solve marches like the others.
+// 4096x512 and 2600 at 16384x1024.  Where the memory for the powers cannot be had,
+// the first solve marches like the others.
 __host__ __device__ constexpr int so_ranges(int L) { return 148 * (L >= 9 ? 1 : L >= 6 || L == 1 ? 2 : 3); }
 constexpr int SO_MAX_RANGES = 148 * 3;
 
@@ -1566,14 +1569,18 @@ sp_first_gram_kernel(const __grid_constant__ SsArgs a, const KoStepState* st) {
         }
     }
     if (!sp_last_block(a)) return;
-    // a power: one and four coefficients in, one out; the sums: all in
-    ss_gram_serial<true>(a, lev, {56.0 * lev[0] + 8.0, 56.0 * lev[1] + 8.0}, [&](double (*tot)[SS_NG]) {
-        for (int s = 0; s < 2; ++s)
-            for (int i = warp; lev[s] > 0 && i < (lev[s] + 1) * (lev[s] + 2) / 2; i += SS_WARPS) {
-                const double v = sum_slot_warp(part[s], so_ranges(lev[s]), i);
-                if (lane == 0) tot[s][i] = v;
-            }
-    });
+    ss_gram_serial<true>(
+        a, [&](int s) { return s ? lev[1] : lev[0]; },
+        // a power: one and four coefficients in, one out; the sums: all in
+        [&](int s) { return 56.0 * (s ? lev[1] : lev[0]) + 8.0; },
+        [&](double (*tot)[SS_NG]) {
+#pragma unroll
+            for (int s = 0; s < 2; ++s)
+                for (int i = warp; lev[s] > 0 && i < (lev[s] + 1) * (lev[s] + 2) / 2; i += SS_WARPS) {
+                    const double v = sum_slot_warp(part[s], so_ranges(lev[s]), i);
+                    if (lane == 0) tot[s][i] = v;
+                }
+        });
 }
 
 // ---- the update on the device -------------------------------------------------------------
