@@ -1,0 +1,41 @@
+"""Orders of memory that no run can show to be missing, looked for in the source.
+
+sstep_kernel and ku_rest_kernel write global arrays and march them in the same
+launch, and march several units whose shared memory is laid out differently.
+Bulk copies (the async proxy) are ordered after ordinary accesses only by a
+proxy fence on the way from the one to the other."""
+import os
+import re
+
+import komegafoulingmodel_b200
+
+CSRC = os.path.join(os.path.dirname(komegafoulingmodel_b200.__file__), "csrc")
+FENCE = "ss_proxy_fence();"
+
+
+def body(name, file="kofm_sstep.cuh"):
+    """The body of a device function, without comments."""
+    text = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, file)).read())
+    at = re.search(r"__device__[^;{}]*\b%s\([^;{}]*\)\s*\{" % name, text)
+    depth, i = 1, at.end()
+    while depth:
+        depth += {"{": 1, "}": -1}.get(text[i], 0)
+        i += 1
+    return text[at.end():i - 1]
+
+
+def test_the_fences_cover_global_and_shared_memory():
+    assert 'asm volatile("fence.proxy.async;" ::: "memory")' in body("ss_proxy_fence")
+    assert 'asm volatile("fence.proxy.async.shared::cta;" ::: "memory")' in body("ss_proxy_fence_shared")
+
+
+def test_grid_barrier_orders_writes_before_later_copies():
+    sync = body("ss_sync")
+    assert FENCE in sync[:sync.index("atomicAdd")], "before the arrival"
+    assert FENCE in sync[sync.rindex("ss_sync_march();"):], "after the wait"
+
+
+def test_a_unit_ends_with_a_fence():
+    march = body("ss_march")
+    assert re.search(r"ss_proxy_fence_shared\(\);\s*ss_sync_march\(\);\s*$", march)
+    assert "ss_proxy_fence_shared();" in body("ss_unit_sums")[-40:]
