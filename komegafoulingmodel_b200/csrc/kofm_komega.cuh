@@ -432,8 +432,10 @@ __device__ __forceinline__ void km_assemble(const AsmParams& p, const double dt,
     // k, omega of rows r-2 .. r (start r = y0 - 1; row y0 - 3 is never used);
     // row r + 1 comes from the ring
     FT k0 = FT(0), o0 = FT(0);
-    FT k1 = __ldg(pK + crow(y0 - 2) * P + cx), o1 = __ldg(pO + crow(y0 - 2) * P + cx);
-    FT k2 = __ldg(pK + crow(y0 - 1) * P + cx), o2 = __ldg(pO + crow(y0 - 1) * P + cx);
+    // (k and omega are not read-only where one launch runs several sub-steps:
+    // no non-coherent loads)
+    FT k1 = __ldcg(pK + crow(y0 - 2) * P + cx), o1 = __ldcg(pO + crow(y0 - 2) * P + cx);
+    FT k2 = __ldcg(pK + crow(y0 - 1) * P + cx), o2 = __ldcg(pO + crow(y0 - 1) * P + cx);
     // flag of row r (loaded one step ahead)
     int t = y0 - 1 >= 0 ? (uint16_t)__ldg(p.ntype + (y0 - 1) * P + cx) : M_SOLID;
     // carried from row r - 1: flag, ring fields, closure

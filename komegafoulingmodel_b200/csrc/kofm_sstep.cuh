@@ -1237,9 +1237,11 @@ __device__ __forceinline__ bool ss_resid_units(const SsArgs& a, const bool act[2
                 const double dS = y > 0 ? __ldcg(S.x + gj - a.P) : 0.0;
                 const double dN = y + 1 < a.ny ? __ldcg(S.x + gj + a.P) : 0.0;
                 // CSR order of an interior row: S, W, C, E, N
-                const double Ad = __ldg(cf + 96) * dS + __ldg(cf + 32) * __ldcg(S.x + row + xw) + __ldcg(S.x + gj) +
-                                  __ldg(cf) * __ldcg(S.x + row + xe) + __ldg(cf + 64) * dN;
-                rr[j] = __ldg(S.rhs + gj) - Ad;
+                // (the rows are not read-only where one launch runs several
+                // sub-steps: no non-coherent loads)
+                const double Ad = __ldcg(cf + 96) * dS + __ldcg(cf + 32) * __ldcg(S.x + row + xw) + __ldcg(S.x + gj) +
+                                  __ldcg(cf) * __ldcg(S.x + row + xe) + __ldcg(cf + 64) * dN;
+                rr[j] = __ldcg(S.rhs + gj) - Ad;
             }
             __stcg(reinterpret_cast<double2*>(S.r + g), make_double2(rr[0], rr[1]));
             acc[0] += rr[0] * rr[0] + rr[1] * rr[1];

@@ -110,3 +110,51 @@ def test_restarts_and_substeps_finish_on_the_device(kofm_lib, krylov, storage):
         q = np.abs(coef.reshape(4, -1)).sum(0).max()
         bound = 4 * 2 * 2 * REL_TOL * np.linalg.norm(rhs) / (1 - q) + 4 * eps * np.abs(a).max()
         assert q < 1 and np.abs(a - b).max() <= bound, (i, q, np.abs(a - b).max(), bound)
+
+
+@pytest.mark.parametrize("nx,ny,krylov,storage", [
+    (300, 43, 2, _abi.STORE_FP64), (96, 26, 3, _abi.STORE_FP64),  # the second: a lattice that stays in L1
+    (300, 43, 10, _abi.STORE_FP64), (300, 43, 3, _abi.STORE_FP32),
+])
+def test_substeps_with_restarts_of_a_wavy_channel_in_one_launch(kofm_lib, nx, ny, krylov, storage):
+    """Both systems' residuals reported as NaN once: four sub-steps, three of them
+    assembled, solved with restarts and applied by the launch that finishes an
+    update, and four more in the step after; against the host-driven rounds, whose
+    assemblies and sweeps are launches of their own.  Bound as above, with the
+    largest right-hand side met and seven solves."""
+    ch = G.wavy_channel(nx, ny, 0.05 * ny, nx // 2)
+    f = perturbed_state(ch, seed=5, u_mean=0.05, rho_amp=1e-4, u_amp=5e-3, neq_amp=1e-5)
+    k, o, nut, s = komega_state(ch, seed=6)
+    got, norms, q = [], [], 0.0
+    for form in (0, 3):
+        d = desc_default()
+        d.nx, d.nx_full, d.ny = nx, nx, ny
+        d.tau, d.fterm, d.mu = 1.0 / (3 * 1e-3 + 0.5), 1e-7, 1e-3
+        d.use_komega, d.storage = 1, storage
+        d.komega_rel_tol, d.komega_abs_tol = REL_TOL, 0.0
+        d.krylov_dim, d.komega_classic = krylov, form
+        d.komega_max_iters = 10000
+        fields = []
+        with Lattice(d) as L:
+            L.set_geometry(ch.ntype, ch.wallD, ch.dX, ch.ibb_idx, ch.ibb_q)
+            L.set_state(f, k, o, nut, s)
+            L.step(2)
+            for fail in (1, 0):
+                if fail:
+                    L.debug_fail_solves(1, mask=3)
+                L.step(1)
+                st = L.stats()
+                assert st.steps_per_lb == 4 and max(st.omega_restarts, st.k_restarts) > 2
+                _, K, O, _, _ = L.get_state()
+                fields += [O, K]
+                for i in (0, 1):
+                    coef, rhs = L.komega_rows(i)
+                    norms.append(np.linalg.norm(rhs))
+                    q = max(q, np.abs(coef.reshape(4, -1)).sum(0).max())
+        got.append(fields)
+    eps = np.finfo(np.float32 if storage == _abi.STORE_FP32 else np.float64).eps
+    assert q < 1
+    for i, (a, b) in enumerate(zip(*got)):
+        rhs = max(norms[i % 2::2])
+        bound = 7 * 2 * 2 * REL_TOL * rhs / (1 - q) + 7 * eps * np.abs(a).max()
+        assert np.abs(a - b).max() <= bound, (i, q, np.abs(a - b).max(), bound)

@@ -39,3 +39,12 @@ def test_a_unit_ends_with_a_fence():
     march = body("ss_march")
     assert re.search(r"ss_proxy_fence_shared\(\);\s*ss_sync_march\(\);\s*$", march)
     assert "ss_proxy_fence_shared();" in body("ss_unit_sums")[-40:]
+
+
+def test_only_constant_arrays_are_read_non_coherently():
+    """k, omega and the rows change within ku_rest_kernel; the flags and the index
+    of the link fractions do not."""
+    for name, file in (("km_assemble", "kofm_komega.cuh"), ("ss_resid_units", "kofm_sstep.cuh"),
+                       ("ss_write_units", "kofm_sstep.cuh"), ("ss_march", "kofm_sstep.cuh")):
+        for args in re.findall(r"__ldg\(([^)]*)", body(name, file)):
+            assert args.startswith(("p.ntype", "p.dxidx")), (name, args)
