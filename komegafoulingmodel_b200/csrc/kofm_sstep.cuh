@@ -242,6 +242,9 @@ __device__ __forceinline__ void ss_gram_begin(const SsArgs& a, GmresSys& S, cons
         const int i = e / n, j = e - i * n;
         cs.G[e] = t[i <= j ? ss_gslot(i, j) : ss_gslot(j, i)];
     }
+    // (a cut by diag(R) indexes R with another stride and meets entries that no
+    // vector writes: they are 0, as in the reference)
+    for (int e = lane + 32 * part; e < a.K * a.K; e += 16 * SS_WARPS) cs.R[e] = 0.0;
     if (part == 0 && lane == 0) {
         const double rho0 = sqrt(t[0]);
         S.powers += L;

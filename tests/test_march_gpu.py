@@ -158,3 +158,46 @@ def test_substeps_with_restarts_of_a_wavy_channel_in_one_launch(kofm_lib, nx, ny
         rhs = max(norms[i % 2::2])
         bound = 7 * 2 * 2 * REL_TOL * rhs / (1 - q) + 7 * eps * np.abs(a).max()
         assert np.abs(a - b).max() <= bound, (i, q, np.abs(a - b).max(), bound)
+
+
+@pytest.mark.parametrize("form", [0, 2, 3])
+def test_cycles_cut_by_the_diagonal_of_r(kofm_lib, form):
+    """A cycle that ends because diag(R) fell below relTol R(0, 0) back-substitutes
+    with R indexed by the vectors kept, where from two on it meets entries that no
+    vector wrote: they are zero, the update is not finite, and the solve reports a
+    NaN residual and leaves the field.  Against the form of one vector per sweep:
+    the same outcome, and the same fields but for the rounding of sums of 12,000
+    products (sqrt(12000) eps = 2.4e-14).  Here omega keeps one vector, k one at
+    0.1 and two at 0.03."""
+    nx, ny = 300, 40
+    ch = G.straight_channel(nx, ny)
+    state = (perturbed_state(ch, seed=3, u_mean=0.05, rho_amp=1e-4, u_amp=5e-3, neq_amp=1e-5),
+             *komega_state(ch, seed=4, s_amp=0.1))
+
+    def solves(form, tol):
+        d = desc_default()
+        d.nx, d.nx_full, d.ny = nx, nx, ny
+        d.tau, d.fterm, d.mu = 1.0 / (3 * 1e-3 + 0.5), 1e-7, 1e-3
+        d.use_komega, d.storage, d.komega_classic = 1, _abi.STORE_FP64, form
+        d.komega_rel_tol, d.komega_abs_tol = tol, 0.0
+        with Lattice(d) as L:
+            L.set_geometry(ch.ntype, ch.wallD, ch.dX)
+            for _ in range(3):  # the later ones meet what the earlier ones left in shared memory
+                L.set_state(*state)
+                L.lb_step()
+                L.komega_assemble(1.0)
+                L.komega_solve(raise_on_error=False)
+                st = L.stats()
+                counts = [(st.omega_iters, st.omega_vectors, st.omega_nan), (st.k_iters, st.k_vectors, st.k_nan)]
+                yield counts, L.get_state()[2:0:-1]
+
+    kept = []
+    for tol in (0.1, 0.03):
+        list(solves(form, 1e-4))  # full cycles: R filled
+        counts, fields = next(solves(1, tol))
+        kept += [iters for iters, vectors, _ in counts if iters == vectors - 1]  # one test of xi fewer: cut by diag(R)
+        for got, got_fields in solves(form, tol):
+            assert got == counts, tol
+            for a, b in zip(got_fields, fields):
+                assert np.abs(a - b).max() <= 1e-13 * np.abs(b).max(), (tol, got)
+    assert kept == [1, 1, 1, 2], kept
