@@ -90,6 +90,12 @@ constexpr double KO_A1 = 0.31, KO_KAPPA = 0.41, KO_C_MU_0_25 = 0.5477225575;
 constexpr double KO_GAMMA1 = 5.0 / 9.0, KO_GAMMA2 = 0.44;
 
 // ---- storage conversions ------------------------------------------------
+// RO: through a read-only load, which the compiler may move above a grid_wait();
+// a kernel that has one reads what its predecessor wrote without (with them and
+// after_wait() on the pointer instead a laminar step of 256x64 took 4.47 us, so
+// 3.84).
+template <bool RO, typename T>
+__device__ __forceinline__ T ld_vec(const T* p) { return RO ? __ldg(p) : *p; }
 template <typename ST> struct Store;
 // vt: the type a population is loaded into and stored from (FP32 for the
 // 32- and 16-bit forms, FP64 for the FP64 form)
@@ -98,9 +104,10 @@ template <> struct Store<double> {
     __device__ static double to_f32(double v) { return v; }
     __device__ static double to_f64(double v) { return v; }
     __device__ static double from_f64(double v) { return v; }
+    template <bool RO>
     __device__ static void load4(const double* p, double o[4]) {
-        const double2 a = __ldg(reinterpret_cast<const double2*>(p));
-        const double2 b = __ldg(reinterpret_cast<const double2*>(p) + 1);
+        const double2 a = ld_vec<RO>(reinterpret_cast<const double2*>(p));
+        const double2 b = ld_vec<RO>(reinterpret_cast<const double2*>(p) + 1);
         o[0] = a.x; o[1] = a.y; o[2] = b.x; o[3] = b.y;
     }
     __device__ static void store4(double* p, const double v[4]) {
@@ -115,8 +122,9 @@ template <> struct Store<float> {
     __device__ static float from_f32(float v) { return v; }
     __device__ static double to_f64(float v) { return (double)v; }
     __device__ static float from_f64(double v) { return (float)v; }
+    template <bool RO>
     __device__ static void load4(const float* p, float o[4]) {
-        float4 v = __ldg(reinterpret_cast<const float4*>(p));
+        float4 v = ld_vec<RO>(reinterpret_cast<const float4*>(p));
         o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w;
     }
     __device__ static void store4(float* p, const float v[4]) {
@@ -129,8 +137,9 @@ template <> struct Store<__half> {
     __device__ static double to_f64(__half v) { return (double)__half2float(v); }
     __device__ static __half from_f32(float v) { return __float2half_rn(v); }
     __device__ static __half from_f64(double v) { return __double2half(v); }
+    template <bool RO>
     __device__ static void load4(const __half* p, float o[4]) {
-        uint2 raw = __ldg(reinterpret_cast<const uint2*>(p));
+        uint2 raw = ld_vec<RO>(reinterpret_cast<const uint2*>(p));
         __half2 a = *reinterpret_cast<__half2*>(&raw.x);
         __half2 b = *reinterpret_cast<__half2*>(&raw.y);
         float2 fa = __half22float2(a), fb = __half22float2(b);
@@ -151,8 +160,9 @@ template <> struct Store<__nv_bfloat16> {
     __device__ static double to_f64(__nv_bfloat16 v) { return (double)__bfloat162float(v); }
     __device__ static __nv_bfloat16 from_f32(float v) { return __float2bfloat16_rn(v); }
     __device__ static __nv_bfloat16 from_f64(double v) { return __double2bfloat16(v); }
+    template <bool RO>
     __device__ static void load4(const __nv_bfloat16* p, float o[4]) {
-        uint2 raw = __ldg(reinterpret_cast<const uint2*>(p));
+        uint2 raw = ld_vec<RO>(reinterpret_cast<const uint2*>(p));
         __nv_bfloat162 a = *reinterpret_cast<__nv_bfloat162*>(&raw.x);
         __nv_bfloat162 b = *reinterpret_cast<__nv_bfloat162*>(&raw.y);
         float2 fa = __bfloat1622float2(a), fb = __bfloat1622float2(b);

@@ -201,13 +201,13 @@ __device__ __forceinline__ void lb_block(const LbParams& p, int bx, int by, int 
         const int cx = cx_of(q), cy = cy_of(q);
         VT v[4];
         if (PHASE0) {
-            Store<ST>::load4(gin + q * D + rowoff + x0, v);
+            Store<ST>::template load4<KOMEGA || NEQ>(gin + q * D + rowoff + x0, v);
         } else {
             int ys = y - cy;
             ys = ys < 0 ? 0 : (ys >= p.ny ? p.ny - 1 : ys);  // only solid rows clamp
             const ST* src = gin + q * D + (long long)ys * p.P;
             VT c[4];
-            Store<ST>::load4(src + x0, c);
+            Store<ST>::template load4<KOMEGA || NEQ>(src + x0, c);
             if (cx == 0) {
                 v[0] = c[0]; v[1] = c[1]; v[2] = c[2]; v[3] = c[3];
             } else if (cx == 1) {

@@ -48,3 +48,20 @@ def test_only_constant_arrays_are_read_non_coherently():
                        ("ss_write_units", "kofm_sstep.cuh"), ("ss_march", "kofm_sstep.cuh")):
         for args in re.findall(r"__ldg\(([^)]*)", body(name, file)):
             assert args.startswith(("p.ntype", "p.dxidx")), (name, args)
+
+
+def test_overlapped_kernels_read_behind_their_wait():
+    """A kernel placed while its predecessor runs: what that one wrote is read
+    through ordinary loads, which stay below the wait, or through a pointer taken
+    behind it."""
+    step = body("lb_block", "kofm_lb.cuh")
+    assert "if constexpr (!KOMEGA && !NEQ) grid_wait();" in open(os.path.join(CSRC, "kofm_lb.cuh")).read()
+    assert re.findall(r"load4<([^>]*)>", step) == ["KOMEGA || NEQ"] * 2
+    # the other read-only loads of the collide: the FP16_NEQ moments, wall distances
+    assert re.findall(r"(\w*ldg\w*)\(", step) == ["fld_ldg4"]
+    text = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, "kofm_adjoint.inc")).read())
+    for name, pointers in (("k_adj_lambda", ("nu", "lam", "sg")), ("k_adj_stream_t", ("lam", "nu", "dq"))):
+        kernel = text[text.index(name + "("):]
+        kernel = kernel[kernel.index("{"):]
+        waits = re.match(r"\{\s*grid_wait\(\);((?:\s*after_wait\(\w+\);)*)", kernel).group(1)
+        assert re.findall(r"\((\w+)\)", waits) == list(pointers), name
