@@ -105,10 +105,12 @@ constexpr double SS_PIVOT_MIN = 1.0e-9;
 // magnitudes of its terms (the Gram entries' own sums over the nodes).
 constexpr double SS_PRED_EPS = 1.0e-13;
 
-// Sum over each half of a warp (every lane of the half gets it).
+// Sum over each half of a warp: every lane of the half gets it, the same to the
+// last bit (an addition that is not fused with the product a caller passes, or
+// two lanes would round it differently and could take different branches).
 __device__ __forceinline__ double ss_sum16(double x) {
 #pragma unroll
-    for (int off = 8; off > 0; off >>= 1) x += __shfl_xor_sync(0xffffffffu, x, off);
+    for (int off = 8; off > 0; off >>= 1) x = __dadd_rn(x, __shfl_xor_sync(0xffffffffu, x, off));
     return x;
 }
 
@@ -192,13 +194,13 @@ __device__ __forceinline__ void ss_cycle(SsCycle& c, SsCycleSmem& cs, int L, int
         double Gw = a0 + a1;
         double h[SS_MAXL];
 #pragma unroll
-        for (int j = 0; j < k; ++j) h[j] = ss_sum16(ORDERED ? __dmul_rn(w, GV[j]) : w * GV[j]);
+        for (int j = 0; j < k; ++j) h[j] = ss_sum16(w * GV[j]);
 #pragma unroll
         for (int j = 0; j < k; ++j) {
             w -= h[j] * c.V[j];
             Gw -= h[j] * GV[j];
         }
-        const double nk2 = ss_sum16(ORDERED ? __dmul_rn(w, Gw) : w * Gw);
+        const double nk2 = ss_sum16(w * Gw);
         double inv, nk;  // a vanishing direction cuts (diag test)
         if (ORDERED) {
             nk = nk2 > 0.0 ? sqrt(nk2) : 0.0;

@@ -1,11 +1,14 @@
-"""Orders of memory that no run can show to be missing, looked for in the source.
+"""What no run can show to be missing, looked for in the source: orders of memory,
+and lanes of a warp that have to agree.
 
 sstep_kernel and ku_rest_kernel write global arrays and march them in the same
 launch, and march several units whose shared memory is laid out differently.
 Bulk copies (the async proxy) are ordered after ordinary accesses only by a
 proxy fence on the way from the one to the other."""
 import os
+import random
 import re
+from fractions import Fraction
 
 import komegafoulingmodel_b200
 
@@ -65,3 +68,18 @@ def test_overlapped_kernels_read_behind_their_wait():
         kernel = kernel[kernel.index("{"):]
         waits = re.match(r"\{\s*grid_wait\(\);((?:\s*after_wait\(\w+\);)*)", kernel).group(1)
         assert re.findall(r"\((\w+)\)", waits) == list(pointers), name
+
+
+def test_lanes_agree_on_what_their_branches_read():
+    """The tests that end a cycle are taken by every lane of a warp from its own
+    copy of a sum over the lanes; with that sum's first addition fused into the
+    product before it, lanes i and j round a_i b_i + a_j b_j differently, and the
+    warp could part at a shuffle that waits for all of it."""
+    def fma(a, b, c):
+        return float(Fraction(a) * Fraction(b) + Fraction(c))
+
+    rng = random.Random(1)
+    draw = [[rng.uniform(0.5, 1.0) for _ in range(4)] for _ in range(100)]
+    assert any(fma(a, b, c * d) != fma(c, d, a * b) for a, b, c, d in draw)
+    assert all(a * b + c * d == c * d + a * b for a, b, c, d in draw)
+    assert "x = __dadd_rn(x, __shfl_xor_sync(0xffffffffu, x, off));" in body("ss_sum16")
