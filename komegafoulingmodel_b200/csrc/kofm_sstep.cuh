@@ -69,7 +69,8 @@ struct SsArgs {
     int maxu;
     GridBarrier* bar;
     SsQueue* queue;
-    int* lhint;               // [2] powers of a first round, kept across solves (0: K)
+    int* lhint;               // powers of a first round, kept across solves (0: K): [2], then [2] of zeros
+                              // for a loaded state's first solve
     int nx, ny, P;
     long long D;
     int K;                    // Krylov dimension
@@ -1503,8 +1504,9 @@ sp_gram_kernel(const __grid_constant__ SsArgs a, const KoStepState* st) {
 // which later steps do not take back.  So that solve takes its sums in one fixed
 // order, whatever the form, the row ranges and the units of a march: the nodes in
 // so_ranges(L) ranges of whole 32-column groups, a thread every 256th node of a
-// range, then the threads of a warp, the warps, the ranges; and its cycle takes
-// the reference's formulas to the letter (ss_cycle<true>).  Measured on 242
+// range, then the threads of a warp, the warps, the ranges.  It takes all K powers,
+// whatever the solves of an earlier state took, and its cycle the reference's
+// formulas to the letter (ss_cycle<true>).  Measured on 242
 // channels with wavy walls, the fields after 6 steps: with the marches' sums 17
 // differ by over 0.8% of omega or k at a node from the fixed order's, by up to
 // 60%; here the three forms agree to 2e-7.
