@@ -61,7 +61,7 @@ struct GmresSys {
     int lev;            // two-sweep cycle: levels of its last Gram sweep
     int ext;            // two-sweep cycle: 1 = more powers needed before the cut
     int powers;         // two-sweep cycle: powers computed (all rounds and cycles)
-    int lnext;          // two-sweep cycle: first-round powers chosen for the next cycle (0: none yet)
+    int lnext;          // two-sweep cycle: first-round powers chosen for the next solve's first cycle (0: none yet)
     // two-sweep cycle: the restart whose residual is in use (0: b'), the levels
     // of the pending Gram sweep (0: none), what the update sweep does
     // (SsApply), a kept correction waiting for its residual sweep, and the

@@ -25,9 +25,10 @@
 // at once.  Where it does not (tight tolerances, or a further restart), the
 // second sweep keeps d, and a residual sweep forms b' - A d and its norm.
 //
-// L follows the cycle lengths seen so far (two more powers than the last
-// cycle used, kept per system across solves); a cycle whose tests have not
-// fired by then is run again with the powers up to the Krylov dimension.
+// L follows the cycle lengths seen so far (two more powers than the last such
+// cycle used, kept per system across solves, for a solve's first cycle and for
+// its later ones, which are shorter); a cycle whose tests have not fired by then
+// is run again with the powers up to the Krylov dimension.
 // In FP64 the truncation tests see rounding of the size the reference's own
 // classical Gram-Schmidt has (both lose orthogonality like eps cond^2), so the
 // cut of a converged cycle moves by a vector or two with the order of a sum, and
@@ -69,8 +70,8 @@ struct SsArgs {
     int maxu;
     GridBarrier* bar;
     SsQueue* queue;
-    int* lhint;               // powers of a first round, kept across solves (0: K): [2], then [2] of zeros
-                              // for a loaded state's first solve
+    int* lhint;               // powers of a cycle's first sweep, kept across solves (0: K): [2] of a solve's
+                              // first cycle, [2] of zeros for a loaded state's first solve, [2] of later cycles
     int nx, ny, P;
     long long D;
     int K;                    // Krylov dimension
@@ -343,8 +344,8 @@ __device__ __forceinline__ void ss_gram_end(const SsArgs& a, GmresSys& S, int s,
         S.vec_index_sum += c.built * (c.built - 1) / 2;
         int nl = c.built + 2;
         nl = nl > K ? K : nl;
-        __stcg(a.lhint + s, nl);
-        S.lnext = nl;
+        __stcg(a.lhint + s + (S.rst ? 4 : 0), nl);
+        if (!S.rst) S.lnext = nl;
         // the next restart's test (GMRESSolver.cpp:248-256), where it is certain
         const int next = S.rst + 1;
         const double thr = fmax(a.rel_tol * S.norm_rhs, a.abs_tol);
@@ -381,7 +382,7 @@ __device__ __forceinline__ void ss_resid_step(const SsArgs& a, GmresSys& S, int 
     else S.cycles += 1;
     S.rst += 1;
     S.ready = 0;
-    S.lto = S.active ? ss_hint_levels(__ldcg(a.lhint + s), a.K) : 0;
+    S.lto = S.active ? ss_hint_levels(__ldcg(a.lhint + 4 + s), a.K) : 0;
     if (!S.active) S.bmode = SS_B_WRITE;
 }
 
