@@ -78,6 +78,7 @@ struct SsArgs {
     int max_restarts;
     double rel_tol, abs_tol;
     long long spin_limit;
+    int launches;             // of an update
     // row ranges a strip is split into, by both systems' level counts + 1 (0: a
     // system with nothing to do): the Gram sweep and the update sweep
     short gram_rows[SS_MAXL + 2][SS_MAXL + 2];
@@ -1475,19 +1476,24 @@ __global__ void sp_init_kernel(GmresControl* ctl, GridBarrier* bar, SsQueue* que
 // (st: the sub-stepping state of the update graph, whose sweeps do nothing once
 // an update has stopped with an error; null in the host-driven form)
 __device__ __forceinline__ bool sp_stopped(const KoStepState* st) { return st && ldc(&st->status) != 0; }
+// A sweep of a further round of the update graph has something to do while the
+// round before asked for it.
+__device__ __forceinline__ bool sp_idle(const KoStepState* st, int further) {
+    return sp_stopped(st) || (further && !ldc(&st->again));
+}
 
 __global__ void __launch_bounds__(SS_THREADS)
-sp_resid_kernel(const __grid_constant__ SsArgs a, const KoStepState* st) {
+sp_resid_kernel(const __grid_constant__ SsArgs a, const KoStepState* st, int further) {
     bool act[2];
-    if (sp_stopped(st)) return;
+    if (sp_idle(st, further)) return;
     ss_resid_pending(a, act);
     if (!ss_resid_units(a, act)) return;
     if (sp_last_block(a)) ss_resid_serial(a, act);
 }
 
 __global__ void __launch_bounds__(SS_BLOCK, 1)
-sp_gram_kernel(const __grid_constant__ SsArgs a, const KoStepState* st) {
-    if (sp_stopped(st)) return;
+sp_gram_kernel(const __grid_constant__ SsArgs a, const KoStepState* st, int further) {
+    if (sp_idle(st, further)) return;
     ss_specialise(a, [&] {
         if (!ss_begin(a, true, ss_gram_levels(a, 0), ss_gram_levels(a, 1))) return;
         ss_gram_unit(a, blockIdx.x);
@@ -1664,11 +1670,27 @@ ku_assemble_kernel(const AsmParams p, GmresControl* ctl, GridBarrier* bar, SsQue
     km_assemble<FT>(p, ku_dt(st), blockIdx.x * KM_WARPS + (threadIdx.x >> 5));
 }
 
-constexpr int KU_LAUNCHES = 4;  // assembly, Gram and update sweep, the rest
+constexpr int KU_LAUNCHES = 4;  // assembly, Gram and update sweep, the rest; three per further round
+// Rounds of a solve that the update enqueues as sweeps of their own after the
+// first, before the kernel for the rest: those that the options make usual.  A
+// cycle ends at 1e-6 to 1e-9 of its start, so below that a second one follows, of
+// few vectors each several; at the default tolerance there is none, and three
+// launches with nothing to do would be 6 us.  The rest kernel has one block per SM
+// and a barrier's wait between sweeps, which a small lattice does not feel.  With
+// rounds left to it and enqueued, us a step at 1e-9, 10 vectors a cycle (one
+// round): 256x64 113 and 119, 1001x253 203 and 186, 4096x512 1054 and 893,
+// 16384x1024 7190 and 5710; 3 vectors (three rounds): 256x64 94 and 116, 2048x256
+// 223 and 231, 4096x512 682 and 665, 16384x1024 5280 and 4870.
+__host__ inline int ku_further_rounds(double rel_tol, int K, long long nodes) {
+    if (rel_tol >= 1.0e-6 && K >= 3) return 0;
+    if (K >= 8) return nodes >= 1 << 17 ? 1 : 0;
+    return nodes >= 1 << 20 ? 3 : 0;
+}
 
 // Decisions after `rounds` rounds of a solve (one thread): what is left of the
 // update.
-__device__ __forceinline__ void ku_round_end(GmresControl* ctl, KoStepState* st, int rounds, int max_rounds) {
+__device__ __forceinline__ void ku_round_end(const SsArgs& a, KoStepState* st, int rounds, int max_rounds) {
+    GmresControl* ctl = a.ctl;
     if (st->fresh) {
         if (ku_doubles(st->time_since_change, st->steps_per_lb)) {
             st->steps_per_lb /= 2;
@@ -1677,8 +1699,8 @@ __device__ __forceinline__ void ku_round_end(GmresControl* ctl, KoStepState* st,
         st->time_since_change = st->time_since_change + 1 >= 20 ? 0 : st->time_since_change + 1;
         st->cur = 0;
         st->substeps = 0;
-        st->launches = KU_LAUNCHES;
-        st->launches_total += KU_LAUNCHES;
+        st->launches = a.launches;
+        st->launches_total += a.launches;
         st->updates++;
         st->fresh = 0;
     }
@@ -1720,14 +1742,14 @@ __device__ __forceinline__ void ku_round_end(GmresControl* ctl, KoStepState* st,
 // The update sweep.
 template <typename FT>
 __global__ void __launch_bounds__(SS_BLOCK, 1)
-sp_update_kernel(const __grid_constant__ SsArgs a, KoStepState* st, int max_rounds) {
-    if (sp_stopped(st)) return;
+sp_update_kernel(const __grid_constant__ SsArgs a, KoStepState* st, int max_rounds, int further) {
+    if (sp_idle(st, further)) return;
     ss_specialise(a, [&] {
         if (ss_begin(a, false, ss_upd_levels(a, 0), ss_upd_levels(a, 1))) ss_upd_unit<FT>(a, blockIdx.x);
         ss_write_units<FT>(a);
         if (sp_last_block(a) && threadIdx.x == 0) {
             ss_upd_serial(a);
-            if (st) ku_round_end(a.ctl, st, 1, max_rounds);
+            if (st) ku_round_end(a, st, 1, max_rounds);
         }
     });
 }
@@ -1752,7 +1774,7 @@ ku_rest_kernel(const __grid_constant__ SsArgs a, const __grid_constant__ AsmPara
                 if (!ss_sync(a, [] {})) break;
             }
             const int rounds = ss_solve<FT>(a);
-            if (!ss_sync(a, [&] { if (threadIdx.x == 0) ku_round_end(a.ctl, st, rounds, max_rounds); })) break;
+            if (!ss_sync(a, [&] { if (threadIdx.x == 0) ku_round_end(a, st, rounds, max_rounds); })) break;
             if (!ldc(&st->go)) return;
         }
         if (threadIdx.x == 0) {  // a barrier's wait ran out

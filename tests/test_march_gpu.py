@@ -201,3 +201,47 @@ def test_cycles_cut_by_the_diagonal_of_r(kofm_lib, form):
             for a, b in zip(got_fields, fields):
                 assert np.abs(a - b).max() <= 1e-13 * np.abs(b).max(), (tol, got)
     assert kept == [1, 1, 1, 2], kept
+
+
+@pytest.mark.parametrize("nx,ny,krylov,restarts", [(600, 220, 10, 3), (1100, 960, 3, 3), (1100, 960, 1, 5)])
+def test_further_rounds_of_an_update(kofm_lib, nx, ny, krylov, restarts):
+    """Lattices and tolerances at which the update's second and later cycles are
+    launches of their own (2^17 nodes with 8 vectors a cycle and more, 2^20 with
+    fewer), with more rounds than those launches (1 vector), fewer (after a step
+    that converges sooner), and sub-steps: the host-driven rounds' fields, the
+    bound as above with eleven solves."""
+    ch = G.straight_channel(nx, ny)
+    f = perturbed_state(ch, seed=3, u_mean=0.05, rho_amp=1e-4, u_amp=5e-3, neq_amp=1e-5)
+    k, o, nut, s = komega_state(ch, seed=4)
+    got, norms, q = [], [], 0.0
+    for form in (0, 3):
+        d = desc_default()
+        d.nx, d.nx_full, d.ny = nx, nx, ny
+        d.tau, d.fterm, d.mu = 1.0 / (3 * 1e-3 + 0.5), 1e-7, 1e-3
+        d.use_komega, d.storage = 1, _abi.STORE_FP64
+        d.komega_rel_tol, d.komega_abs_tol = REL_TOL, 0.0
+        d.krylov_dim, d.komega_classic = krylov, form
+        d.komega_max_iters = 10000
+        fields = []
+        with Lattice(d) as L:
+            L.set_geometry(ch.ntype, ch.wallD, ch.dX)
+            L.set_state(f, k, o, nut, s)
+            for fail in (0, 0, 1, 0):
+                if fail:
+                    L.debug_fail_solves(1, mask=3)
+                L.step(1)
+                st = L.stats()
+                assert max(st.omega_restarts, st.k_restarts) >= restarts
+                _, K, O, _, _ = L.get_state()
+                fields += [O, K]
+                for i in (0, 1):
+                    coef, rhs = L.komega_rows(i)
+                    norms.append(np.linalg.norm(rhs))
+                    q = max(q, np.abs(coef.reshape(4, -1)).sum(0).max())
+            assert st.steps_per_lb == 4
+        got.append(fields)
+    assert q < 1
+    for i, (a, b) in enumerate(zip(*got)):
+        rhs = max(norms[i % 2::2])
+        bound = 11 * 2 * 2 * REL_TOL * rhs / (1 - q) + 11 * np.finfo(float).eps * np.abs(a).max()
+        assert np.abs(a - b).max() <= bound, (i, q, np.abs(a - b).max(), bound)
