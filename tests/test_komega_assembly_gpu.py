@@ -115,3 +115,34 @@ def test_chunk_length_does_not_change_the_rows(kofm_lib, ny, repeat):
     for one, many in zip(*out):
         assert np.isfinite(one).all() and np.any(one)
         assert np.array_equal(np.tile(one, (1, 1, repeat)), many)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("storage", [_abi.STORE_FP32, _abi.STORE_FP64])
+@pytest.mark.parametrize("ny,repeat", [(253, 17), (253, 30), (34, 137)])
+def test_chunk_length_does_not_change_the_rows_beside_curved_walls(kofm_lib, storage, ny, repeat):
+    """The same with wavy walls of period 60, whose nodes take the weights of uneven
+    links, and in both types."""
+    nx, mu = 60, 5e-4
+    ch = G.wavy_channel(nx, ny, 0.1 * ny, nx)
+    state = (perturbed_state(ch, seed=3, u_mean=0.03), *komega_state(ch, seed=4, k0=4e-5, o0=2e-3, s_amp=2e-4))
+    assert (ch.dX != 1.0).any()
+    out = []
+    for m in (1, repeat):
+        def tiled(a):
+            return np.tile(np.reshape(a, (-1, ny, nx)), (1, 1, m)).ravel()
+
+        d = desc_default()
+        d.nx, d.nx_full, d.ny = nx * m, nx * m, ny
+        d.tau, d.fterm, d.mu = 1.0 / (3 * mu + 0.5), 0.0, mu
+        d.use_komega, d.storage = 1, storage
+        with Lattice(d) as L:
+            L.set_geometry(tiled(ch.ntype), tiled(ch.wallD), tiled(ch.dX))
+            L.set_state(*map(tiled, state))
+            L.lb_step()
+            L.komega_assemble(1.0)
+            out.append([np.concatenate([c.reshape(4, ny, nx * m), r.reshape(1, ny, nx * m)])
+                        for c, r in map(L.komega_rows, range(2))])
+    for one, many in zip(*out):
+        assert np.isfinite(one).all() and np.any(one)
+        assert np.array_equal(np.tile(one, (1, 1, repeat)), many)
