@@ -1355,6 +1355,10 @@ __device__ __forceinline__ void ss_specialise(const SsArgs& a, F body) {
     ss_sync_march();
     if (threadIdx.x == 0) ss_sm().go = 0;
     ss_sync_block();
+    // After a wait that ran out, copies may be in flight into this block's shared
+    // memory: it stays for a while (1 ms, far above a copy's time) before it ends.
+    if (*(volatile int*)&ss_sm().dead)
+        for (int i = 0; i < 1000; ++i) __nanosleep(1000);
 }
 
 // (returns the rounds run)

@@ -83,3 +83,11 @@ def test_lanes_agree_on_what_their_branches_read():
     assert any(fma(a, b, c * d) != fma(c, d, a * b) for a, b, c, d in draw)
     assert all(a * b + c * d == c * d + a * b for a, b, c, d in draw)
     assert "x = __dadd_rn(x, __shfl_xor_sync(0xffffffffu, x, off));" in body("ss_sum16")
+
+
+def test_a_block_outlives_the_copies_of_a_failed_wait():
+    """A wait that ran out may leave bulk copies in flight into the block's shared
+    memory; the block ends only some time after its last one."""
+    end = body("ss_specialise")
+    end = end[end.rindex("ss_sync_block();"):]
+    assert re.search(r"if \(\*\(volatile int\*\)&ss_sm\(\)\.dead\)\s*for \(int i = 0; i < 1000; \+\+i\) __nanosleep\(1000\);", end)
