@@ -519,6 +519,22 @@ __global__ void k_shear_links(const double* __restrict__ tau_nodes, const int32_
     out[b] = acc;
 }
 
+// Whether a loaded state's first solve takes its sums in their fixed order
+// (sp_first_gram_kernel): where its right-hand side is large beside omega, that
+// is where a wall passes a node nearer than half way to it (the wall's omega is
+// 6 nu / (0.075 d^2), at most 1000) or omega is above 1000.  On straight half-way
+// walls (d = 1/2) it never was: the fields agree to 4e-7 with any order, and the
+// first step keeps its time (16384x1024 2.6 ms less, of an end-to-end run of 20
+// steps 2.5%).
+template <typename FT>
+__global__ void k_first_ordered(const FT* __restrict__ wallD, const FT* __restrict__ omega,
+                                const int16_t* __restrict__ ntype, int* flag, int nx, int P) {
+    const int x = blockIdx.x * blockDim.x + threadIdx.x;
+    const long long g = (long long)blockIdx.y * P + x;
+    const bool here = x < nx && !(ntype[g] & M_SOLID) && (!(wallD[g] >= FT(0.25)) || !(fabs(omega[g]) <= FT(1000)));
+    if (__syncthreads_or(here) && threadIdx.x == 0 && *(volatile int*)flag == 0) atomicExch(flag, 1);
+}
+
 // FP64 host-layout scalar field <-> device field (FP32, or FP64 in the FP64 form)
 template <typename FT>
 __global__ void k_field_in(const double* __restrict__ h, FT* __restrict__ dv, int nxf,
@@ -1032,6 +1048,14 @@ int kofm_set_state(kofm_ctx* c, const double* f, const double* k, const double* 
         for (int s = 0; s < 3; ++s)
             if ((st = upload_field(c, sxy + s * Dh, field_plane(c, c->S, s)))) return st;
     }
+    if (d.use_komega) {
+        int* flag = reinterpret_cast<int*>(c->red_out);
+        KOFM_CUDA_TRY(cudaMemsetAsync(flag, 0, sizeof(int), c->stream), KOFM_ERR_MEMORY_COPY);
+        if (c->f64) k_first_ordered<double><<<grid, 128, 0, c->stream>>>((const double*)c->wallD, (const double*)c->O, c->ntype, flag, d.nx, c->P);
+        else k_first_ordered<float><<<grid, 128, 0, c->stream>>>((const float*)c->wallD, (const float*)c->O, c->ntype, flag, d.nx, c->P);
+        KOFM_CUDA_TRY(cudaGetLastError(), KOFM_ERR_CALLING_KERNEL);
+        KOFM_CUDA_TRY(cudaMemcpyAsync(c->h_red, flag, sizeof(int), cudaMemcpyDeviceToHost, c->stream), KOFM_ERR_MEMORY_COPY);
+    }
     KOFM_CUDA_TRY(cudaStreamSynchronize(c->stream), KOFM_ERR_MEMORY_COPY);
     c->phase = 0;
     c->have_state = true;
@@ -1042,10 +1066,10 @@ int kofm_set_state(kofm_ctx* c, const double* f, const double* k, const double* 
     if (c->steps_per_lb < 1) c->steps_per_lb = 1;
     c->time_since_change = 0;
     if (d.use_komega) {
+        c->first_solve = *reinterpret_cast<const int*>(c->h_red) != 0;
         ug_pull(c);  // updates still in flight finish first
         ug_reset(c);
-        c->first_solve = true;
-        first_solve_alloc(c);
+        if (c->first_solve) first_solve_alloc(c);
         c->launches_host = 0;
         c->stats.solver_launches_total = 0;
     }

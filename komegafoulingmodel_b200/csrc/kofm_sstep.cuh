@@ -441,13 +441,13 @@ __device__ __forceinline__ void sp_sys_store(GmresControl* ctl, int s, const Gmr
 // The step loop is unrolled so that all register windows are circular buffers
 // with compile-time slots: level j's row y stays in registers until the Gram
 // sums of row y are formed (L - j steps later); the compiler keeps each value
-// exactly that long.  From 8 levels on, the registers keep three rows and the
+// exactly that long.  From 7 levels on, the registers keep three rows and the
 // older values wait in shared memory (the far history).
 
 // Dynamic shared memory of a march: the ring, the rows that the threads'
 // x neighbours read (the newest values of two levels side by side, per step
 // parity, one column more on each side), and the far history of a Gram sweep
-// of 8 and more levels (one column per thread).
+// of 7 and more levels (one column per thread).
 __host__ __device__ constexpr int ss_row_bytes() { return (SS_THREADS + 2) * 16; }
 __host__ __device__ constexpr int ss_nb_bytes(int L) { return 2 * ((L + 1) / 2) * ss_row_bytes(); }
 constexpr int SS_FAR = 7;  // levels from which a Gram sweep keeps a far history
@@ -1520,12 +1520,13 @@ sp_gram_kernel(const __grid_constant__ SsArgs a, const KoStepState* st, int furt
 // formulas to the letter (ss_cycle<true>).  Measured on 242
 // channels with wavy walls, the fields after 6 steps: with the marches' sums 17
 // differ by over 0.8% of omega or k at a node from the fixed order's, by up to
-// 60%; here the three forms agree to 2e-7.
+// 60%; with these sums the largest difference is 5e-6 (1e-7 the median).
 //
 // The powers are formed one after the other in memory and summed in a pass of
 // their own: a loaded state's first step takes 80 us more at 256x64, 350 at
-// 4096x512 and 2600 at 16384x1024.  Where the memory for the powers cannot be had,
-// the first solve marches like the others.
+// 4096x512 and 2600 at 16384x1024, so only states that need it take it
+// (k_first_ordered).  Where the memory for the powers cannot be had, the first
+// solve marches like the others.
 __host__ __device__ constexpr int so_ranges(int L) { return 148 * (L >= 9 ? 1 : L >= 6 || L == 1 ? 2 : 3); }
 constexpr int SO_MAX_RANGES = 148 * 3;
 

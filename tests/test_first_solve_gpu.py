@@ -86,3 +86,24 @@ def test_cycles_end_as_recorded_in_every_form(kofm_lib, nx, ny):
                 bound = np.finfo(np.float32).eps * np.abs(b) + 64 * np.finfo(float).eps * np.abs(start).max()
                 assert np.all(np.abs(a - b) <= bound), (amp, np.abs(a - b).max())
     assert not wrong, wrong
+
+
+@pytest.mark.parametrize("amp,omega,powers", [(0.0, None, 0), (0.0, 2e3, 10), (3.0, None, 10)])
+def test_states_that_need_the_fixed_order_take_it(kofm_lib, amp, omega, powers):
+    """Straight half-way walls need none; a node near a wall, or omega above the wall
+    rows' cap anywhere, does.  Seen in the launches: a first solve in the fixed
+    order has one per power and one for the sums, where a march has one."""
+    nx, ny = 301, 66
+    nu, yb, yt, state = _start(nx, ny, amp)
+    if omega:
+        state[2][(ny // 2) * nx + 7] = omega
+    d = desc_default()
+    d.nx, d.nx_full, d.ny, d.komega_classic = nx, nx, ny, 3
+    d.tau, d.fterm, d.mu, d.use_komega = 1.0 / (3 * nu + 0.5), 1e-7, nu, 1
+    with Lattice(d) as L:
+        L.set_walls(yb, yt)
+        L.set_state(*state)
+        L.step(1)
+        L.sync()
+        st = L.stats()
+        assert st.solver_launches == 3 * st.solver_rounds + powers
