@@ -130,10 +130,13 @@ typedef struct kofm_desc {
                                  restart cycle, as GMRESSolver::solve does;
                                  0 (default): end the cycle as soon as its
                                  truncation tests fire (see kofm_komega_solve) */
-    int32_t solver_max_blocks;/* cap on the k-omega solver's grid (0: two
-                                 blocks per SM, fewer on small lattices);
-                                 lattices advanced together (kofm_batch_*)
-                                 may share the GPU better with a cap */
+    int32_t solver_max_blocks;/* cap on the k-omega solver's grid (0: one block
+                                 per SM; form 1 two per SM, fewer on small
+                                 lattices); the sweeps that are launches of
+                                 their own are split for that many, at least
+                                 one per strip of columns; lattices advanced
+                                 together (kofm_batch_*) may share the GPU
+                                 better with a cap */
     /* thermal implicit FD (clVariablesFD::loadParams, clVariablesFD.cpp:444-493) */
     int32_t use_thermal;      /* thermalSolverFlag (USE_THERMAL_SOLVER) */
     int32_t thermal_every;    /* tfdSteps: LB steps per thermal update
@@ -196,8 +199,9 @@ typedef struct kofm_stats {
                                            array its sweeps stream, counted once per sweep */
     int32_t omega_powers, k_powers;     /* two-sweep cycles: powers of the Gram sweeps (all rounds) */
     int32_t solver_launches;            /* kernel launches of the last k-omega solve */
-    int32_t solver_rounds;              /* rounds of the last solve (phase launches:
-                                           powers + Gram + update sweeps; 1 otherwise) */
+    int32_t solver_rounds;              /* rounds of the last solve (Gram and update
+                                           sweep, from the second on a residual sweep
+                                           first; 1 for the one-launch forms) */
     int64_t solver_launches_total;      /* kernel launches of all k-omega updates
                                            since the state was loaded */
 } kofm_stats;
