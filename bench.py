@@ -163,7 +163,7 @@ def replica_value(nodes: int, steps: int, world: int, ms: float) -> float:
 SOLVER_TRAFFIC_RATIO = {
     "gmres_kernel": 4.7967e9 / (1076 * 4194304),   # one vector per sweep
     "sstep_kernel": None,                          # two sweeps per cycle
-    "sstep_phases": None,                          # the same, one launch per sweep
+    "sstep_phases": 937.7e6 / (220 * 4194304),     # the same, one launch per sweep
 }
 
 STORE_BYTES = {"fp32": 4, "fp16": 2, "bf16": 2, "fp16neq": 2, "fp16neq32": 2, "fp16row": 2, "fp64": 8}
