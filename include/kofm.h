@@ -277,7 +277,10 @@ int kofm_get_geometry(kofm_ctx* ctx, int16_t* ntype, double* wallD, double* dX4,
  * nut may be NULL (it is recomputed by the next step).  Replaces the
  * allocate_buffer_w_copy uploads of ini() and the lbf/lbkappa/lbomega bin
  * loads (clVariablesLB.cpp:883-902, kOmega.cpp:685-710); as there, the
- * k-omega sub-stepping starts again from the descriptor's komega_dt. */
+ * k-omega sub-stepping starts again from the descriptor's komega_dt.  A state
+ * with a node nearer than 1/4 to a wall, or with omega above 1000, takes
+ * 16 krylov_dim bytes a node for the sums of its first solve, where they can be
+ * had (kept with the context). */
 int kofm_set_state(kofm_ctx* ctx, const double* f, const double* k,
                    const double* omega, const double* nut, const double* sxy);
 
